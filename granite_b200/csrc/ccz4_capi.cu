@@ -31,10 +31,10 @@ using namespace granite_b200;
 namespace granite_b200 {
 
 // Tensor map of one block buffer for the TMA stage kernel: 4-D (x, y, z,
-// field) over the cells incl. ghosts, FP64, box = 16 x 4 x tz tile + 4-cell
-// halo, no swizzle, zero fill outside the block. The driver's encoder is looked
+// field) over the cells incl. ghosts, FP64, the box of a shape (ccz4_kernels.h),
+// no swizzle, zero fill outside the block. The driver's encoder is looked
 // up once through the runtime (no link against libcuda).
-bool encode_block_tmap(void* map128, const double* base, const DevBlock& d, int tz) {
+bool encode_block_tmap(void* map128, const double* base, const DevBlock& d, int shape) {
     static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
     static std::once_flag once;
     std::call_once(once, [] {
@@ -50,12 +50,14 @@ bool encode_block_tmap(void* map128, const double* base, const DevBlock& d, int 
     if (!encode || !base) return false;
     // global address 16-byte aligned, every stride a multiple of 16 bytes (x extent even)
     if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || (d.tx & 1) != 0) return false;
-    const int bz = tz + 8;
-    if (d.tx < TMA_BOX_X || d.ty < TMA_BOX_Y || d.tz < bz) return false;
+    const int tz = TMA_SHAPE_TZ[shape];  // (0 for the far planes)
+    if (d.tx < TMA_BOX_X || d.ty < TMA_BOX_Y || d.tz < tz + 8) return false;
+    const bool arm = shape == TMA_SHAPE_ARM;
     const cuuint64_t dims[4] = {(cuuint64_t)d.tx, (cuuint64_t)d.ty, (cuuint64_t)d.tz, (cuuint64_t)NV};
     const cuuint64_t strides[3] = {(cuuint64_t)d.tx * sizeof(double), (cuuint64_t)d.tx * d.ty * sizeof(double),
                                    (cuuint64_t)d.stride * sizeof(double)};
-    const cuuint32_t box[4] = {(cuuint32_t)TMA_BOX_X, (cuuint32_t)TMA_BOX_Y, (cuuint32_t)bz, 1};
+    const cuuint32_t box[4] = {(cuuint32_t)(arm ? TMA_ARM_X : TMA_BOX_X), (cuuint32_t)(arm ? TMA_ARM_Y : TMA_BOX_Y),
+                               (cuuint32_t)(arm ? TMA_ARM_Z : tz + 2), 1};
     const cuuint32_t estride[4] = {1, 1, 1, 1};
     const CUresult r = encode(static_cast<CUtensorMap*>(map128), CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4,
                               const_cast<double*>(base), dims, strides, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -68,13 +70,16 @@ bool encode_block_tmap(void* map128, const double* base, const DevBlock& d, int 
 
 namespace {
 
-// Stage configuration per (precision: FP64, MIXED) and block-size class
-// (GRANITE_STAGE_CLASS_EDGES) until a caller sets its own: the autotuner's
-// (granite_b200/tuner.py) uniform table on a B200, one configuration per
-// precision, so a level stage stays one launch. Mixed: configuration 12
-// (x-remainder tiles) has the least total over the classes, its 19-23 % gain
-// on blocks 8 cells wider than a multiple of 16 outweighing 1-3 % elsewhere.
-constexpr int DEFAULT_CLASS_CFG[2][GRANITE_STAGE_CLASSES] = {{0, 0, 0, 0, 0, 0}, {12, 12, 12, 12, 12, 12}};
+// The configuration granite_ccz4_get_stage_config reports for a class without
+// one of its own; which tile set a level then runs is level_default_tileset's
+// choice.
+constexpr int DEFAULT_CFG = 12;
+
+// A table entry or forced configuration that leaves the choice to the library.
+constexpr int AUTO_CFG = -1;
+
+// The tile set of the per-block drop-in (the one with the store epilogue).
+constexpr int STORE_TILESET = 0;
 
 static_assert(sizeof(CUtensorMap) == 128, "tensor maps are 128 bytes");
 static_assert(alignof(CUtensorMap) >= 64, "tensor maps are 64-byte aligned");
@@ -87,9 +92,9 @@ struct Graph {
     long long launches = 0;
 };
 
-// Tiles of one stage-kernel configuration within a level's work-list: one launch.
+// Tiles of one TMA tile set within a level's work-list: one launch.
 struct StageGroup {
-    int cfg;          // TMA configuration (TMA_CFGS), 0 for the other variants
+    int tileset;      // 0 for the other variants
     int first, count; // range of the level's tiles
 };
 
@@ -97,12 +102,14 @@ struct LevelLists {
     std::vector<int> blocks;
     int variant = VARIANT_GLOBAL;  // stage kernel of this level: the context's variant, or GLOBAL
                                    // when a block cannot be mapped for TMA
-    // stage-kernel tiles: per precision (0 FP64, 1 MIXED) grouped by
-    // configuration (groups), each block's tiles contiguous (tile_range)
+    // stage-kernel tiles: per precision (0 FP64, 1 MIXED) grouped by tile
+    // set (groups), each block's tiles contiguous (tile_range)
     Tile* d_tiles = nullptr;
     std::vector<Tile> h_tiles;       // host copy of d_tiles (push lists are built from it)
     std::vector<StageGroup> groups[2];
-    std::vector<int> block_cfg[2];  // per block of the level: its configuration
+    std::vector<int> block_tiles[2];  // per block of the level: its tile set
+    // every block has the same stencil coefficients (one spacing, to the last bit)
+    bool uniform = true;
     int ntiles = 0;
     unsigned char* d_flags = nullptr;  // per-tile precision of MIXED steps (1 = FP64 algebra)
     Tile* d_mtiles = nullptr;  // constraint-monitor tiles (variant-0 shape)
@@ -218,7 +225,7 @@ struct Ctx {
     std::vector<char> step_pushed;
     unsigned long long* d_cmp = nullptr; // granite_ccz4_compare_states results (46 words)
     CUtensorMap* d_tmaps = nullptr;      // TMA variant: per box shape, 3 maps per resident block (slots 0-2)
-    CUtensorMap* s_tmap = nullptr;       // TMA variant: map of the stateless single-block input
+    CUtensorMap* s_tmap = nullptr;       // TMA variant: the two maps of the stateless single-block input
 
     // stateless scratch (grow-only)
     double* s_u = nullptr;
@@ -316,6 +323,11 @@ DevBlock make_devblock(const granite_block_desc& b, double sigma) {
     d.inv4hh[0] = 1.0 / (4.0 * d.dx[0] * d.dx[1]);
     d.inv4hh[1] = 1.0 / (4.0 * d.dx[0] * d.dx[2]);
     d.inv4hh[2] = 1.0 / (4.0 * d.dx[1] * d.dx[2]);
+    for (int a = 0; a < 3; ++a) {
+        d.inv12h_f[a] = (float)d.inv12h[a];
+        d.inv12h2_f[a] = (float)d.inv12h2[a];
+        d.inv4hh_f[a] = (float)d.inv4hh[a];
+    }
     d.level = b.level;
     return d;
 }
@@ -323,11 +335,10 @@ DevBlock make_devblock(const granite_block_desc& b, double sigma) {
 // Tiles of one block. adaptive (global-load stage kernels only): pick the tile
 // width w in {32, 16, 8} (128 / w rows) that leaves the fewest idle threads on
 // this block's x-y face, preferring the wider tile on ties (longer coalesced rows).
-// rem_mapped: the block has tensor maps of its configuration's remainder box.
 void tiles_of(int block, const granite_block_desc& b, std::vector<Tile>& out, int variant, bool adaptive = false,
-              int cfg = 0, bool rem_mapped = false) {
+              int tileset = 0) {
     int TX, TY, TZ;
-    stage_tile_dims(variant, cfg, &TX, &TY, &TZ);
+    stage_tile_dims(variant, &TX, &TY, &TZ);
     int w = 0;
     if (adaptive) {
         long long best = -1;
@@ -347,8 +358,7 @@ void tiles_of(int block, const granite_block_desc& b, std::vector<Tile>& out, in
     // TMA x-remainder tiles: a block whose x extent is TMA_REM_X more than a
     // multiple of 16 covers its last TMA_REM_X columns with TMA_REM_X x TY x 2 TZ
     // tiles (Tile::w = -TMA_REM_X), each after the full tiles of its rows
-    const bool rem = variant == VARIANT_TMA && !adaptive && cfg >= 0 && cfg < NUM_TMA_CFGS && TMA_CFGS[cfg].rem &&
-                     rem_mapped && b.ncells[0] % TX == TMA_REM_X;
+    const bool rem = variant == VARIANT_TMA && tileset == 1 && b.ncells[0] % TX == TMA_REM_X;
     const int nx = rem ? b.ncells[0] - TMA_REM_X : b.ncells[0];
     for (int k = 0; k < b.ncells[2]; k += TZ)
         for (int j = 0; j < b.ncells[1]; j += TY) {
@@ -369,6 +379,22 @@ int stage_class_of(const granite_block_desc& b) {
     return best;
 }
 
+// The default tile set of a level, one for all its blocks so that a stage is
+// one launch: with x-remainder tiles where they save more tiles than their
+// larger ring slots cost. Per point-stage of a block without remainder columns
+// they take 3.5 % (mixed, 355 against 343 us on 128 x 128 x 64 points) and 3 %
+// (FP64, 484 against 470) longer; a block of width 24 has a quarter fewer tiles.
+int level_default_tileset(const Ctx* c, const std::vector<int>& blocks) {
+    long long n[NUM_TMA_TILESETS] = {};
+    for (int i : blocks)
+        for (int q = 0; q < NUM_TMA_TILESETS; ++q) {
+            std::vector<Tile> t;
+            tiles_of(i, c->descs[i], t, VARIANT_TMA, false, q);
+            n[q] += (long long)t.size();
+        }
+    return n[1] * 1.035 < n[0] ? 1 : 0;
+}
+
 long long ghost_count(const granite_block_desc& b) {
     return cells_of(b) - (long long)b.ncells[0] * b.ncells[1] * b.ncells[2];
 }
@@ -378,7 +404,16 @@ void ghost_chunks_of(int block, const granite_block_desc& b, std::vector<GhostIt
     for (long long r = 0; r < n; r += 256) out.push_back(GhostItem{block, (int)r});
 }
 
-// TMA configuration of a block for precision index pr (0 FP64, 1 MIXED).
+// Whether two blocks have the same stencil coefficients, bit for bit.
+bool same_coef(const StencilCoef& a, const StencilCoef& b) {
+    for (int d = 0; d < 3; ++d)
+        if (a.inv12h[d] != b.inv12h[d] || a.inv12h2[d] != b.inv12h2[d] || a.inv4hh[d] != b.inv4hh[d] ||
+            a.kocf[d] != b.kocf[d])
+            return false;
+    return true;  // (kow and the float copies are functions of these)
+}
+
+// TMA configuration the caller set for a block and precision index pr (0 FP64, 1 MIXED), or AUTO_CFG.
 int block_cfg(const Ctx* c, int pr, const granite_block_desc& b) {
     if (c->forced_cfg >= 0) return c->forced_cfg;
     return c->class_cfg[pr][stage_class_of(b)];
@@ -441,16 +476,16 @@ int stage_single(Ctx* c, const granite_block_desc* b, double* u_dev, int* ntiles
     if (r) return r;
     DevBlock d = make_devblock(*b, c->p.ko_sigma);
     d.buf[0] = u_dev ? u_dev : c->s_u;
-    if (variant == VARIANT_TMA) {  // configuration 0 (the one with the store epilogue)
-        CUtensorMap m;
-        if (encode_block_tmap(&m, d.buf[0], d, TMA_CFGS[0].tz))
-            CK(cudaMemcpyAsync(c->s_tmap, &m, sizeof(m), cudaMemcpyHostToDevice, s), "upload tensor map");
+    if (variant == VARIANT_TMA) {
+        CUtensorMap m[2];
+        if (encode_block_tmap(&m[0], d.buf[0], d, 0) && encode_block_tmap(&m[1], d.buf[0], d, TMA_SHAPE_ARM))
+            CK(cudaMemcpyAsync(c->s_tmap, m, sizeof(m), cudaMemcpyHostToDevice, s), "upload tensor maps");
         else
             variant = VARIANT_GLOBAL;
     }
     if (used) *used = variant;
     std::vector<Tile> t;
-    tiles_of(0, *b, t, variant);
+    tiles_of(0, *b, t, variant, false, STORE_TILESET);
     if ((r = ensure_scratch(c, (size_t)cells_of(*b), (int)t.size()))) return r;
     CK(cudaMemcpyAsync(c->s_desc, &d, sizeof(d), cudaMemcpyHostToDevice, s), "upload block descriptor");
     CK(cudaMemcpyAsync(c->s_tiles, t.data(), t.size() * sizeof(Tile), cudaMemcpyHostToDevice, s), "upload tiles");
@@ -562,7 +597,7 @@ int granite_ccz4_set_stage_config(void* h, int precision, int cls, int cfg) {
     if (cfg < -1 || cfg >= NUM_TMA_CFGS) return fail(c, GRANITE_ERR_INVALID, "unknown stage configuration");
     const int pr = precision == GRANITE_PRECISION_MIXED ? 1 : 0;
     for (int q = 0; q < GRANITE_STAGE_CLASSES; ++q)
-        if (cls < 0 || q == cls) c->class_cfg[pr][q] = cfg < 0 ? DEFAULT_CLASS_CFG[pr][q] : cfg;
+        if (cls < 0 || q == cls) c->class_cfg[pr][q] = cfg < 0 ? AUTO_CFG : cfg;
     return GRANITE_OK;
 }
 
@@ -571,6 +606,7 @@ int granite_ccz4_get_stage_config(const void* h, int precision, int cls, int* cf
     if (!c || !cfg || cls < 0 || cls >= GRANITE_STAGE_CLASSES) return GRANITE_ERR_INVALID;
     if (precision != GRANITE_PRECISION_FP64 && precision != GRANITE_PRECISION_MIXED) return GRANITE_ERR_INVALID;
     *cfg = c->forced_cfg >= 0 ? c->forced_cfg : c->class_cfg[precision == GRANITE_PRECISION_MIXED ? 1 : 0][cls];
+    if (*cfg == AUTO_CFG) *cfg = DEFAULT_CFG;
     return GRANITE_OK;
 }
 
@@ -679,7 +715,8 @@ int granite_ccz4_create(const granite_ccz4_params* p, void** out) {
     if (cudaGetDeviceProperties(&prop, p->device) != cudaSuccess) return GRANITE_ERR_NO_DEVICE;
     if (prop.major != 10) return GRANITE_ERR_NO_DEVICE;  // kernels are built for sm_100a only
     Ctx* c = new Ctx();
-    std::memcpy(c->class_cfg, DEFAULT_CLASS_CFG, sizeof(c->class_cfg));
+    for (auto& row : c->class_cfg)
+        for (int& k : row) k = AUTO_CFG;
     c->p = *p;
     c->device = p->device;
     cudaError_t e = cudaSetDevice(c->device);
@@ -692,7 +729,7 @@ int granite_ccz4_create(const granite_ccz4_params* p, void** out) {
     if (e == cudaSuccess) e = cudaMemset(c->d_nonfinite, 0, sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMalloc(&c->d_errflag, sizeof(unsigned int));
     if (e == cudaSuccess) e = cudaMemset(c->d_errflag, 0, sizeof(unsigned int));
-    if (e == cudaSuccess) e = cudaMalloc(&c->s_tmap, sizeof(CUtensorMap));
+    if (e == cudaSuccess) e = cudaMalloc(&c->s_tmap, 2 * sizeof(CUtensorMap));
     if (e == cudaSuccess) e = cudaMalloc(&c->s_desc, sizeof(DevBlock));
     if (e == cudaSuccess) e = cudaMalloc(&c->s_sum, 2 * sizeof(double));
     if (e != cudaSuccess) {
@@ -844,7 +881,10 @@ int granite_ccz4_compute_rhs_device(void* h, const granite_block_desc* b, const 
     a.Sij = Sij;
     a.S = S;
     a.tmaps = c->s_tmap;  // block 0, slot 0
-    CK(launch_stage(variant, 0, precision, EPI_STORE, c->s_desc, c->s_tiles, nt, a, s), "launch RHS");
+    a.tmaps_arm = c->s_tmap + 1;
+    a.coef_uniform = 1;
+    a.coef = make_devblock(*b, c->p.ko_sigma);
+    CK(launch_stage(variant, STORE_TILESET, precision, EPI_STORE, c->s_desc, c->s_tiles, nt, a, s), "launch RHS");
     c->launches += 1;
     return GRANITE_OK;
 }
@@ -1105,23 +1145,17 @@ static int build_lists(Ctx* c) {
     int maxlev = 0;
     for (const auto& d : c->descs) maxlev = std::max(maxlev, d.level);
     // TMA variant: one tensor map per (box shape, block, slot); a block that
-    // cannot be mapped in the tile shapes (tz = 4 and 2) sends its whole level
-    // to the global-load kernel; a block without the tz = 8 shape (less than 8
-    // cells deep) only goes without the remainder tiles of tz = 4 configurations
+    // cannot be mapped sends its whole level to the global-load kernel
     const size_t nb = c->descs.size();
     std::vector<char> mapped(nb, 0);
-    std::vector<std::array<char, TMA_SHAPES>> shape_ok(nb);
     if (c->variant == VARIANT_TMA) {
         std::vector<CUtensorMap> maps(TMA_SHAPES * 3 * nb);
         for (size_t i = 0; i < nb; ++i) {
-            for (int sh = 0; sh < TMA_SHAPES; ++sh) {
-                bool ok = true;
+            bool ok = true;
+            for (int sh = 0; sh < TMA_SHAPES && ok; ++sh)
                 for (int sl = 0; sl < 3; ++sl)
-                    ok = ok && encode_block_tmap(&maps[(sh * nb + i) * 3 + sl], c->hblocks[i].buf[sl], c->hblocks[i],
-                                                 TMA_SHAPE_TZ[sh]);
-                shape_ok[i][sh] = ok;
-            }
-            mapped[i] = shape_ok[i][tma_shape_for_tz(4)] && shape_ok[i][tma_shape_for_tz(2)];
+                    ok = ok && encode_block_tmap(&maps[(sh * nb + i) * 3 + sl], c->hblocks[i].buf[sl], c->hblocks[i], sh);
+            mapped[i] = ok;
         }
         CK(upload_vec(maps, &c->d_tmaps, c->stream), "upload tensor maps");
     }
@@ -1136,22 +1170,25 @@ static int build_lists(Ctx* c) {
             if (c->descs[i].level == L && c->variant == VARIANT_TMA && !mapped[i]) ll.variant = VARIANT_GLOBAL;
         for (size_t i = 0; i < c->descs.size(); ++i)
             if (c->descs[i].level == L) ll.blocks.push_back((int)i);
-        // per precision: stage tiles grouped by configuration (one launch per
-        // group), each block's tiles contiguous
+        for (int i : ll.blocks) ll.uniform = ll.uniform && same_coef(c->hblocks[i], c->hblocks[ll.blocks[0]]);
+        // per precision: stage tiles grouped by tile set (one launch per group),
+        // each block's tiles contiguous
+        const int auto_tiles = ll.variant == VARIANT_TMA ? level_default_tileset(c, ll.blocks) : 0;
         for (int pr = 0; pr < 2; ++pr) {
-            for (int i : ll.blocks) ll.block_cfg[pr].push_back(ll.variant == VARIANT_TMA ? block_cfg(c, pr, c->descs[i]) : 0);
+            for (int i : ll.blocks) {
+                const int cfg = block_cfg(c, pr, c->descs[i]);
+                ll.block_tiles[pr].push_back(ll.variant != VARIANT_TMA ? 0 : cfg == AUTO_CFG ? auto_tiles : tma_tileset(cfg));
+            }
             ll.tile_range[pr].assign(ll.blocks.size(), {0, 0});
-            for (int cfg = 0; cfg < NUM_TMA_CFGS; ++cfg) {
+            for (int ts = 0; ts < NUM_TMA_TILESETS; ++ts) {
                 const int g0 = (int)tiles.size();
                 for (size_t q = 0; q < ll.blocks.size(); ++q) {
-                    if (ll.block_cfg[pr][q] != cfg) continue;
+                    if (ll.block_tiles[pr][q] != ts) continue;
                     const int t0 = (int)tiles.size();
-                    const int rs = ll.variant == VARIANT_TMA ? tma_rem_shape_of(cfg) : -1;
-                    tiles_of(ll.blocks[q], c->descs[ll.blocks[q]], tiles, ll.variant, adaptive_tiles(ll.variant), cfg,
-                             rs >= 0 && shape_ok[ll.blocks[q]][rs]);
+                    tiles_of(ll.blocks[q], c->descs[ll.blocks[q]], tiles, ll.variant, adaptive_tiles(ll.variant), ts);
                     ll.tile_range[pr][q] = {t0, (int)tiles.size() - t0};
                 }
-                if ((int)tiles.size() > g0) ll.groups[pr].push_back({cfg, g0, (int)tiles.size() - g0});
+                if ((int)tiles.size() > g0) ll.groups[pr].push_back({ts, g0, (int)tiles.size() - g0});
             }
         }
         for (size_t q = 0; q < ll.blocks.size(); ++q) {
@@ -1421,24 +1458,27 @@ int granite_ccz4_download_block(void* h, int i, double* host) {
 // then the FP32 kernel over the unflagged tiles and the FP64 kernel over the
 // flagged ones. The two passes write disjoint tiles, so the in-place last
 // stage is safe and no tile is computed twice.
-static cudaError_t stage_range(Ctx* c, LevelLists& L, int cfg, int precision, const StageArgs& a0, int first,
-                               int count, long long* n) {
+// block >= 0: the tiles are that block's alone, else the blocks of the level.
+static cudaError_t stage_range(Ctx* c, LevelLists& L, int tileset, int precision, const StageArgs& a0, int first,
+                               int count, long long* n, int block = -1) {
     const Tile* tiles = L.d_tiles + first;
     StageArgs a = a0;
-    if (L.variant == VARIANT_TMA) {  // the tensor maps of this configuration's box shape(s)
-        a.tmaps = c->d_tmaps + (size_t)tma_shape_of(cfg) * 3 * c->descs.size();
-        a.tmaps_rem = TMA_CFGS[cfg].rem ? c->d_tmaps + (size_t)tma_rem_shape_of(cfg) * 3 * c->descs.size() : nullptr;
+    a.coef_uniform = block >= 0 || L.uniform;
+    a.coef = c->hblocks[block >= 0 ? block : L.blocks[0]];
+    if (L.variant == VARIANT_TMA) {  // the tensor maps of the box shapes
+        const size_t shape = 3 * c->descs.size();
+        a.tmaps = c->d_tmaps;
+        a.tmaps_rem = c->d_tmaps + TMA_SHAPE_REM * shape;
+        a.tmaps_arm = c->d_tmaps + TMA_SHAPE_ARM * shape;
     }
     if (a.tile_push) a.tile_push += first;  // indexed like the launch's tiles
-    // (the TMA kernel keeps a CTA's selected tiles in shared memory: bounded count)
-    const bool split = precision == GRANITE_PRECISION_MIXED && c->fp64_chi > 0.0 &&
-        (L.variant != VARIANT_TMA || (long long)count <= (long long)tma_grid(cfg) * TMA_SEL_CAP);
+    const bool split = precision == GRANITE_PRECISION_MIXED && c->fp64_chi > 0.0;
     if (!split) {
         ++*n;
-        return launch_stage(L.variant, cfg, precision, EPI_RK, c->d_blocks, tiles, count, a, c->stream);
+        return launch_stage(L.variant, tileset, precision, EPI_RK, c->d_blocks, tiles, count, a, c->stream);
     }
     unsigned char* flags = L.d_flags + first;
-    cudaError_t e = launch_classify(L.variant, cfg, c->d_blocks, tiles, 0, count, a.in_sel, c->fp64_chi, flags,
+    cudaError_t e = launch_classify(L.variant, c->d_blocks, tiles, 0, count, a.in_sel, c->fp64_chi, flags,
                                     c->stream);
     if (e != cudaSuccess) return e;
     StageArgs b = a;
@@ -1452,13 +1492,13 @@ static cudaError_t stage_range(Ctx* c, LevelLists& L, int cfg, int precision, co
     b64.want_prec = 1;
     b.want_prec = 0;
     if (c->profiling || !c->overlap_passes) {
-        if ((e = launch_stage(L.variant, cfg, PM_MIXED, EPI_RK, c->d_blocks, tiles, count, b, c->stream))) return e;
-        return launch_stage(L.variant, cfg, PM_FP64F, EPI_RK, c->d_blocks, tiles, count, b64, c->stream);
+        if ((e = launch_stage(L.variant, tileset, PM_MIXED, EPI_RK, c->d_blocks, tiles, count, b, c->stream))) return e;
+        return launch_stage(L.variant, tileset, PM_FP64F, EPI_RK, c->d_blocks, tiles, count, b64, c->stream);
     }
     if ((e = cudaEventRecord(c->ev_fork, c->stream))) return e;
     if ((e = cudaStreamWaitEvent(c->stream2, c->ev_fork, 0))) return e;
-    if ((e = launch_stage(L.variant, cfg, PM_FP64F, EPI_RK, c->d_blocks, tiles, count, b64, c->stream2))) return e;
-    if ((e = launch_stage(L.variant, cfg, PM_MIXED, EPI_RK, c->d_blocks, tiles, count, b, c->stream))) return e;
+    if ((e = launch_stage(L.variant, tileset, PM_FP64F, EPI_RK, c->d_blocks, tiles, count, b64, c->stream2))) return e;
+    if ((e = launch_stage(L.variant, tileset, PM_MIXED, EPI_RK, c->d_blocks, tiles, count, b, c->stream))) return e;
     if ((e = cudaEventRecord(c->ev_join, c->stream2))) return e;
     return cudaStreamWaitEvent(c->stream, c->ev_join, 0);
 }
@@ -1470,7 +1510,7 @@ static cudaError_t level_stage(Ctx* c, LevelLists& L, int precision, const Stage
     if (c->batched) {
         for (const auto& g : L.groups[pr]) {
             cudaError_t e = timed(c, GRANITE_KERNEL_STAGE,
-                                  [&] { return stage_range(c, L, g.cfg, precision, a, g.first, g.count, n); });
+                                  [&] { return stage_range(c, L, g.tileset, precision, a, g.first, g.count, n); });
             if (e != cudaSuccess) return e;
         }
         return cudaSuccess;
@@ -1478,7 +1518,7 @@ static cudaError_t level_stage(Ctx* c, LevelLists& L, int precision, const Stage
     for (size_t q = 0; q < L.tile_range[pr].size(); ++q) {
         const auto& r = L.tile_range[pr][q];
         cudaError_t e = timed(c, GRANITE_KERNEL_STAGE, [&] {
-            return stage_range(c, L, L.block_cfg[pr][q], precision, a, r.first, r.second, n);
+            return stage_range(c, L, L.block_tiles[pr][q], precision, a, r.first, r.second, n, L.blocks[q]);
         });
         if (e != cudaSuccess) return e;
     }
@@ -1844,7 +1884,7 @@ int build_ghosts_mode(Ctx* c) {
                 for (int pr = 0; pr < 2; ++pr)
                     for (const StageGroup& g : ll.groups[pr]) {
                         int TX, TY, TZ;
-                        stage_tile_dims(ll.variant, g.cfg, &TX, &TY, &TZ);
+                        stage_tile_dims(ll.variant, &TX, &TY, &TZ);
                         const int tdim[3] = {TX, TY, TZ};
                         for (int t = g.first; t < g.first + g.count; ++t) {
                             const Tile& tl = ll.h_tiles[t];

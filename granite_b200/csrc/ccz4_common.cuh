@@ -21,19 +21,25 @@ enum Var : int {
     KTR, GHX, GHY, GHZ, THETA, ALPHA, BETAX, BETAY, BETAZ
 };
 
+// Stencil coefficients of a block, computed once on the host as the reference
+// computes them; the float copies are the doubles rounded once (the mixed form).
+struct StencilCoef {
+    double inv12h[3];    // 1/(12 dx)      first derivative (ccz4.cpp:72)
+    double inv12h2[3];   // 1/(12 dx^2)    second derivative (ccz4.cpp:158)
+    double inv4hh[3];    // 1/(4 dx_a dx_b) mixed (xy, xz, yz) (ccz4.cpp:188)
+    double kocf[3];      // sigma/(64 dx)  KO (ccz4.cpp:886-887)
+    double kow[3][4];    // kocf[d] * {1, -6, 15, -20}: the KO weights of ccz4.cpp:921
+    float inv12h_f[3], inv12h2_f[3], inv4hh_f[3];
+};
+
 // Block descriptor as the kernels see it (one per block, in device memory).
-struct DevBlock {
+struct DevBlock : StencilCoef {
     double* buf[3];      // state, stage A, stage B (slot 0/1/2)
     int n[3];            // interior cells
     int tx, ty, tz;      // cells incl. ghosts
     long long stride;    // cells per field
     double lo[3];
     double dx[3];
-    double inv12h[3];    // 1/(12 dx)      first derivative (ccz4.cpp:72)
-    double inv12h2[3];   // 1/(12 dx^2)    second derivative (ccz4.cpp:158)
-    double inv4hh[3];    // 1/(4 dx_a dx_b) mixed (xy, xz, yz) (ccz4.cpp:188)
-    double kocf[3];      // sigma/(64 dx)  KO (ccz4.cpp:886-887)
-    double kow[3][4];    // kocf[d] * {1, -6, 15, -20}: the KO weights of ccz4.cpp:921
     int level;
     int moff;            // resident matter: cell offset of the block in the context's matter arrays
 };
@@ -62,9 +68,6 @@ struct PushBox {
     int tx, txy;
     int lo[3], hi[3];
 };
-// Push boxes of one tile staged in shared memory by the TMA stage kernel
-// (more than this many: read from global memory).
-constexpr int PUSH_STAGE_MAX = 16;
 
 // Arguments of one fused RHS launch.
 struct StageArgs {
@@ -82,10 +85,16 @@ struct StageArgs {
     unsigned long long* nonfinite;  // floor hits on non-finite chi/alpha (nullable)
     const void* tmaps;     // TMA variant: CUtensorMap of (block b, slot s) at tmaps[3 b + s]
     const void* tmaps_rem; // TMA variant with x-remainder tiles: the same for their box shape
+    const void* tmaps_arm; // TMA variant: the same for the boxes of far z planes
     unsigned int* errflag; // TMA variant: set to 1 when a bounded mbarrier wait gives up (nullable)
     // Per-tile precision (nullable): the launch covers only tiles ti with tile_prec[ti] == want_prec.
     const unsigned char* tile_prec;
     int want_prec;
+    // coef_uniform: every block of the launch has the stencil coefficients `coef`
+    // (the TMA variant then takes them from the kernel arguments), else each
+    // block's own are read from its descriptor
+    int coef_uniform;
+    StencilCoef coef;
     // Test switch of the TMA variant, 0 = off: CTA 0 never issues ring item
     // test_withhold - 1, so its bounded wait for that item runs out (no copy is
     // in flight for it) and the launch reports through errflag.

@@ -12,42 +12,33 @@ enum { EPI_STORE = 0, EPI_RK = 1 };
 // Kernel variants of the fused stage: 0 = stencils from global memory
 // (32x4x1 tiles), 1 = fields staged through shared memory with cp.async
 // (16x4x2 tiles); 2, 3 = variant 0 with the registers capped at 168 / 128 per
-// thread (3 / 4 CTAs per SM); 4 = persistent CTAs that stream every field of
-// a 16x4x4 tile and its halo into a ring of shared-memory slots with TMA
-// (cp.async.bulk.tensor) and mbarriers. The constraint and KO kernels always
+// thread (3 / 4 CTAs per SM); 4 = persistent CTAs whose load warps stream every
+// field of a 16x4x2 tile and its halo into rings of shared-memory slots with
+// TMA (cp.async.bulk.tensor) and mbarriers. The constraint and KO kernels always
 // use variant-0 tiles.
 enum {
     VARIANT_GLOBAL = 0, VARIANT_SMEM = 1, VARIANT_GLOBAL_R168 = 2, VARIANT_GLOBAL_R128 = 3, VARIANT_TMA = 4,
     NUM_VARIANTS = 5
 };
 
-// Tile shape of a stage-kernel variant (points per CTA along x, y, z); cfg
-// selects the TMA configuration.
-int stage_tile_dims(int variant, int cfg, int* tx, int* ty, int* tz);
+// Tile shape of a stage-kernel variant (points along x, y, z).
+void stage_tile_dims(int variant, int* tx, int* ty, int* tz);
 
-// Configurations of the TMA variant (the autotuner's candidates): tiles of
-// 16 x 4 x tz points (tz * 64 threads per CTA; tz = 2 asks for two resident
-// CTAs per SM), a ring of nbuf field boxes; tin: the stage input's centre values
-// are kept in shared memory for the RK epilogue and the epilogue's u^n and the
-// next tile's pointwise cells are prefetched into L2; hs: the Hessian-field
-// loop's 36 values live in shared memory instead of local memory.
-// ws: the mixed RK kernels are warp-specialized (stencil warps feed algebra
-// warps through shared memory; ccz4_stage_ws.cuh), the FP64 ones those of
-// configuration 4. Configuration 0 is the only one with the store (drop-in
-// RHS) epilogue; the defaults per precision and block-size class are in
-// ccz4_capi.cu (DEFAULT_CLASS_CFG).
+// The table of configuration ids of the TMA variant: what a caller may set per
+// precision and block-size class, and what granite_ccz4_stage_config_info tells
+// of each. They were the candidates of the kernel that issued its own loads (its
+// tile depth, ring slots, shared-memory options, CTAs per SM and barrier
+// grouping). The kernel with load warps (ccz4_stage_tma.cuh) is faster than the
+// best of them for every block size and precision (mixed 343 against 411 us,
+// FP64 470 against 501 on 128 x 128 x 64 points), so an id now chooses between
+// its two tile sets only (tma_tileset): x-remainder tiles or not.
 struct TmaCfg {
-    int tz, nbuf, tin, hs, ws;
-    int minb;  // resident CTAs per SM the register allocation is sized for (__launch_bounds__)
-    int bar;   // ring items per CTA barrier (1 or 2; the barrier frees that many slots)
-    // x-remainder tiles: a block whose x extent leaves 8 cells after its
-    // 16-wide tiles covers them with 8 x 4 x 2tz tiles (Tile::w = -8, every
-    // thread on a point) instead of 16-wide tiles half outside the block;
-    // rem = 1 loads them with the 24 x 12 x (2tz + 8) box shape (ring slots
-    // sized for it), rem = 2 as two boxes of the configuration's own shape (one
-    // per half along z, two ring items; needs bar = 2)
+    int tz, nbuf, tin, hs, ws, minb, bar;
+    // x-remainder tiles: a block whose x extent leaves 8 cells after its 16-wide
+    // tiles covers them with 8 x 4 x 4 tiles (Tile::w = -8, every thread on a
+    // point) instead of 16-wide tiles half outside the block
     int rem;
-    int pf;  // L2 prefetches of u^n and the next tile's pointwise cells without tin (tin implies them)
+    int pf;
 };
 constexpr int NUM_TMA_CFGS = 18;
 constexpr TmaCfg TMA_CFGS[NUM_TMA_CFGS] = {
@@ -57,38 +48,32 @@ constexpr TmaCfg TMA_CFGS[NUM_TMA_CFGS] = {
     {2, 4, 0, 0, 0, 2, 2, 0, 0}, {4, 4, 0, 0, 0, 1, 2, 0, 0}, {2, 3, 1, 0, 0, 2, 1, 1, 0},
     {2, 3, 0, 0, 0, 2, 1, 1, 0}, {2, 2, 1, 0, 0, 2, 1, 1, 0}, {2, 3, 0, 0, 0, 2, 1, 1, 1},
     {4, 4, 0, 0, 0, 1, 2, 1, 0}, {4, 4, 0, 0, 0, 1, 2, 2, 0}, {2, 4, 0, 0, 0, 2, 2, 2, 0}};
+// Tile sets of the TMA kernel: 0 = 16 x 4 x 2 tiles (and the store epilogue of the
+// drop-in RHS), 1 = with x-remainder tiles.
+constexpr int NUM_TMA_TILESETS = 2;
+constexpr int tma_tileset(int cfg) { return TMA_CFGS[cfg].rem ? 1 : 0; }
+constexpr int TMA_TZ = 2;
 // Points of an x-remainder tile along x.
 constexpr int TMA_REM_X = 8;
-// The box (cells incl. the 4-cell halo) one tensor-map load brings in per
-// field: 24 x 12 x (tz + 8). Tensor maps exist per box shape: shape 0 (tz =
-// 4), shape 1 (tz = 2) and shape 2 (tz = 8, the remainder tiles of tz = 4
-// configurations; a block less than 8 cells deep has none, and its tz = 4
-// remainder columns keep 16-wide tiles).
+// The boxes three tensor-map loads bring in per field of a tile of depth tz:
+// 24 x 12 x (tz + 2) cells, the tile with its 4-cell halo in x and y and the one
+// plane beyond it on either side in z that the mixed derivatives read off the
+// axes; and, below and above it, 16 x 4 x 3, the farther planes, which the z
+// stencils read at the tile's own columns only. One 24 x 12 x (tz + 8) box would
+// hold 1.6 (tz = 4) or 1.9 (tz = 2) times the cells: as much more shared memory
+// per ring slot and L2 traffic per field.
+// Tensor maps exist per box shape: shape 0 (tz = 2), shape 1 (tz = 4, the
+// remainder tiles) and shape 2, the far planes of every tile.
 constexpr int TMA_BOX_X = 16 + 8, TMA_BOX_Y = 4 + 8;
+constexpr int TMA_ARM_X = 16, TMA_ARM_Y = 4, TMA_ARM_Z = 3;
 constexpr int TMA_SHAPES = 3;
-constexpr int TMA_SHAPE_TZ[TMA_SHAPES] = {4, 2, 8};
-constexpr int tma_shape_for_tz(int tz) { return tz == 4 ? 0 : (tz == 2 ? 1 : (tz == 8 ? 2 : -1)); }
-constexpr int tma_shape_of(int cfg) { return tma_shape_for_tz(TMA_CFGS[cfg].tz); }
-// box shape of a configuration's x-remainder tiles (-1: none)
-constexpr int tma_rem_shape_of(int cfg) {
-    return TMA_CFGS[cfg].rem == 1 ? tma_shape_for_tz(2 * TMA_CFGS[cfg].tz)
-                                  : (TMA_CFGS[cfg].rem == 2 ? tma_shape_of(cfg) : -1);
-}
-// Per-tile precision launches of the TMA kernel keep each CTA's selected tiles
-// in shared memory: at most TMA_SEL_CAP per CTA, i.e. ntiles <= grid x TMA_SEL_CAP.
-constexpr int TMA_SEL_CAP = 1024;
-// Grid of the FP64 pass of the per-tile precision, in resident grids (on the
-// bench hierarchy 1: 76 us per level-stage, 4: 63 us, 8: 55 us, 16: 61 us, the
-// scans of the CTAs without a selected tile outweighing the spread).
-constexpr int TMA_FP64_SPREAD = 8;
-// The resident grid of a TMA configuration's per-tile precision passes on the
-// current device, the smaller of the two (0 before configure_stage_kernels).
-int tma_grid(int cfg);
+constexpr int TMA_SHAPE_TZ[TMA_SHAPES] = {TMA_TZ, 2 * TMA_TZ, 0};
+constexpr int TMA_SHAPE_REM = 1, TMA_SHAPE_ARM = 2;
 // Tensor map of one 22-field block buffer (dims x, y, z, field; cells incl.
-// ghosts) with the box of tile depth tz. Returns false when the buffer cannot
-// be described (odd x extent, misaligned base, box larger than the block);
-// such blocks use the global-load kernel.
-bool encode_block_tmap(void* map128, const double* base, const DevBlock& d, int tz);
+// ghosts) with box shape `shape`. Returns false when the buffer cannot be
+// described (odd x extent, misaligned base) or the block is smaller than a tile
+// with its halo; such blocks use the global-load kernel.
+bool encode_block_tmap(void* map128, const double* base, const DevBlock& d, int shape);
 
 // Per-device kernel attributes (shared-memory opt-in); call with the device current.
 cudaError_t configure_stage_kernels();
@@ -100,15 +85,15 @@ cudaError_t configure_stage_kernels();
 enum { PM_FP64 = 0, PM_MIXED = 1, PM_FP64F = 2 };
 
 // Fused RHS (+KO) over a tile work-list in precision mode `precision` (PM_*);
-// with args.tile_prec set, only the tiles flagged args.want_prec. cfg: the TMA
-// configuration (ignored by the other variants); args.tmaps must hold the
-// tensor maps of that configuration's box shape.
-cudaError_t launch_stage(int variant, int cfg, int precision, int epi, const DevBlock* blocks,
+// with args.tile_prec set, only the tiles flagged args.want_prec. tileset: the
+// TMA tile set (ignored by the other variants); args.tmaps* must hold the tensor
+// maps of its box shapes.
+cudaError_t launch_stage(int variant, int tileset, int precision, int epi, const DevBlock* blocks,
                          const Tile* tiles, int ntiles, const StageArgs& args, cudaStream_t stream);
 
 // Per-tile precision flags of tiles [first, first + ntiles): flag[ti] = 1 when a
 // point of the tile has chi < chi_fp64 in slot `sel` (FP64 algebra), else 0.
-cudaError_t launch_classify(int variant, int cfg, const DevBlock* blocks, const Tile* tiles, int first, int ntiles,
+cudaError_t launch_classify(int variant, const DevBlock* blocks, const Tile* tiles, int first, int ntiles,
                             int sel, double chi_fp64, unsigned char* flag, cudaStream_t stream);
 
 // KO dissipation only: rhs += KO(u) at interior points of one block.

@@ -20,11 +20,10 @@
 // conformal metric, the 1/chi factors, the evolved state and the RK3 combine
 // stay FP64.
 //
-// A stencil source S provides der<HESS, EXACT>(v, beta, w), the derivatives of
-// field v, called for the fields in FIELD_ORDER; S::HS says whether it also
-// provides per-thread shared-memory slots (hess_slots, stride S::NT) for the
-// values of the Hessian-field loop, and S::UNROLL whether that loop may be
-// unrolled (a source whose der() is short).
+// A stencil source S provides der<HESS, EXACT, KOSEP>(v, advec), the derivatives
+// of field v (KOSEP false: advection and KO may come as one sum), called for the
+// fields in FIELD_ORDER, and coefs(), the block's stencil coefficients; UNROLL:
+// the field loops but the first are unrolled.
 #pragma once
 
 #include <type_traits>
@@ -56,16 +55,15 @@ __device__ __forceinline__ bool tile_selected(const unsigned char* prec, int wan
 // evaluates the stencils of one field in the precision of the caller's algebra
 // (P = double or float, deduced from the blend weight w).
 struct GlobalSource {
-    static constexpr bool HS = false;      // the Hessian-field loop's values stay in (local) registers
-    static constexpr bool UNROLL = false;  // and the loop stays rolled (stencil code is long)
+    static constexpr bool UNROLL = true;
     const DevBlock& B;
     const double* __restrict__ u;
     long long c;
-    template <bool HESS, bool EXACT, typename P>
-    __device__ __forceinline__ FieldDer<P> der(int v, const double beta[3], P w) {
-        const long long off[3] = {1, B.tx, (long long)B.tx * B.ty};
-        return field_der_l<P, HESS, true, GlobalLoad, EXACT>(B, GlobalLoad{u + (long long)v * B.stride + c}, off,
-                                                             beta, w);
+    __device__ __forceinline__ const StencilCoef& coefs() const { return B; }
+    template <bool HESS, bool EXACT, bool KOSEP, typename P>
+    __device__ __forceinline__ FieldDer<P> der(int v, const Advection<P, EXACT>& adv) {
+        return field_der_l<P, HESS, true, EXACT, KOSEP>(
+            B, GlobalLoad{u + (long long)v * B.stride + c, {1, B.tx, (long long)B.tx * B.ty}}, adv);
     }
 };
 
@@ -82,20 +80,11 @@ __device__ __forceinline__ void ccz4_point(const DevBlock& B, const double* __re
     // ---- pointwise state (FP64) -------------------------------------------
     const double chi_raw = __ldg(FP(CHI));
     const double chi = (isfinite(chi_raw) && chi_raw >= 1.0e-4) ? chi_raw : 1.0e-4;  // :279-280
-    const double alpha_d = __ldg(FP(ALPHA));
-    const double K_d = __ldg(FP(KTR));
-    const double Th_d = __ldg(FP(THETA));
-    double gtd[6], Atd[6], Ghd[3], beta[3];
+    double gtd[6], beta[3];
 #pragma unroll
-    for (int a = 0; a < 6; ++a) {
-        gtd[a] = __ldg(FP(GXX + a));
-        Atd[a] = __ldg(FP(AXX + a));
-    }
+    for (int a = 0; a < 6; ++a) gtd[a] = __ldg(FP(GXX + a));
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        Ghd[a] = __ldg(FP(GHX + a));
-        beta[a] = __ldg(FP(BETAX + a));
-    }
+    for (int a = 0; a < 3; ++a) beta[a] = __ldg(FP(BETAX + a));
     // inverse conformal metric, FP64 (ccz4.cpp:318-330)
     double gtud[6];
     {
@@ -109,71 +98,65 @@ __device__ __forceinline__ void ccz4_point(const DevBlock& B, const double* __re
         gtud[4] = (gtd[1] * gtd[2] - gtd[0] * gtd[4]) * inv;
         gtud[5] = (gtd[0] * gtd[3] - gtd[1] * gtd[1]) * inv;
     }
-    const P w = (P)(0.5 * (1.0 + tanh((chi - A.chi_c) / A.chi_w)));  // :565
-    const P alpha = (P)alpha_d, K = (P)K_d, Theta = (P)Th_d;
-    P gt[6], At[6], gtu[6], Gh[3];
+    const Advection<P, EXACT> advec(S.coefs(), beta, 0.5 * (1.0 + tanh((chi - A.chi_c) / A.chi_w)));  // :565
+    P gt[6], gtu[6], bp[3];
 #pragma unroll
     for (int a = 0; a < 6; ++a) {
         gt[a] = (P)gtd[a];
-        At[a] = (P)Atd[a];
         gtu[a] = (P)gtud[a];
     }
 #pragma unroll
-    for (int a = 0; a < 3; ++a) Gh[a] = (P)Ghd[a];
+    for (int a = 0; a < 3; ++a) bp[a] = (P)beta[a];
 
     // ---- conformal metric: gradients, Hessian term of Ricci, advection ----
     P dg[6][3];     // d_k gt_ij
     P Rt[6];        // conformal Ricci (ccz4.cpp:465-516), accumulated term by term
-    P agt[6], kgt[6];  // advection and KO of gt
-    // Kept as a loop (one copy of the Hessian-field stencil code instead of
-    // six): the per-point body is otherwise longer than the instruction caches
-    // hold, and instruction fetch stalls the warps. The 36 values it produces
-    // go to this thread's column of shared memory when the source provides one
-    // (Src::HS: slot q of the thread at hs[q * Src::NT]), else to an array in
-    // L1-cached local memory.
-    P* hs = nullptr;
-    if constexpr (Src::HS) {
-        hs = S.template hess_slots<P>();
-        constexpr int T = Src::HS ? Src::NT : 1;
+    // The fields of one tensor go through a loop (one copy of their stencil code
+    // instead of three to seven): unrolled, the per-point body is longer than the
+    // instruction cache holds and instruction fetch stalls the warps. What the
+    // loops produce goes to this thread's scratch, an array in L1-cached local
+    // memory: 36 values, and 12 more where advection and KO are separate (the
+    // reference's order, EXACT).
+    P sc[EXACT ? 48 : 36];
+    // (Src::UNROLL: the loops after the first are unrolled, with their values in
+    // registers; the global-load kernels, whose stencils are short of neither
+    // registers nor instruction fetch but of load latency, are 17 % faster so)
+    constexpr int U3 = Src::UNROLL ? 3 : 1, U7 = Src::UNROLL ? 7 : 1;
+    P sm_[Src::UNROLL ? 48 : 1];
+    P* const sm = Src::UNROLL ? sm_ : sc;
+    // slots: 0-17 the gradients of the loop at hand, 18-23 Rt, then advection (in
+    // the pair form with KO) and KO of gt, Gamma-hat and the shift
+    constexpr int S_RT = 18, S_AG = 24, S_AGH = 30, S_AB = 33, S_KG = 36, S_KGH = 42, S_KB = 45;
+    auto with_ko = [&](P rhs, int slot) {
+        if constexpr (EXACT)
+            return rhs + (slot < S_KGH ? sc[slot] : sm[slot]);
+        else
+            return rhs;
+    };
 #pragma unroll 1
-        for (int a = 0; a < 6; ++a) {
-            FieldDer<P> fd = S.template der<true, EXACT>(GXX + a, beta, w);
+    for (int a = 0; a < 6; ++a) {
+        FieldDer<P> fd = S.template der<true, EXACT, false>(GXX + a, advec);
 #pragma unroll
-            for (int d = 0; d < 3; ++d) hs[(3 * a + d) * T] = fd.d[d];
-            hs[(18 + a) * T] = (P)-0.5 * (gtu[0] * fd.h[0] + gtu[3] * fd.h[3] + gtu[5] * fd.h[5] +
-                                          (P)2 * (gtu[1] * fd.h[1] + gtu[2] * fd.h[2] + gtu[4] * fd.h[4]));
-            hs[(24 + a) * T] = fd.adv;
-            hs[(30 + a) * T] = fd.ko;
-        }
-#pragma unroll
-        for (int a = 0; a < 6; ++a)
-#pragma unroll
-            for (int d = 0; d < 3; ++d) dg[a][d] = hs[(3 * a + d) * T];
-    } else if constexpr (Src::UNROLL) {
-        // a source that evaluates no stencils has a short loop body: unrolled, in registers
-#pragma unroll
-        for (int a = 0; a < 6; ++a) {
-            FieldDer<P> fd = S.template der<true, EXACT>(GXX + a, beta, w);
-#pragma unroll
-            for (int d = 0; d < 3; ++d) dg[a][d] = fd.d[d];
-            Rt[a] = (P)-0.5 * (gtu[0] * fd.h[0] + gtu[3] * fd.h[3] + gtu[5] * fd.h[5] +
-                               (P)2 * (gtu[1] * fd.h[1] + gtu[2] * fd.h[2] + gtu[4] * fd.h[4]));
-            agt[a] = fd.adv;
-            kgt[a] = fd.ko;
-        }
-    } else {
-#pragma unroll 1
-        for (int a = 0; a < 6; ++a) {
-            FieldDer<P> fd = S.template der<true, EXACT>(GXX + a, beta, w);
-#pragma unroll
-            for (int d = 0; d < 3; ++d) dg[a][d] = fd.d[d];
-            // term 1: -1/2 gtu^{lm} d_l d_m gt_ij
-            Rt[a] = (P)-0.5 * (gtu[0] * fd.h[0] + gtu[3] * fd.h[3] + gtu[5] * fd.h[5] +
-                               (P)2 * (gtu[1] * fd.h[1] + gtu[2] * fd.h[2] + gtu[4] * fd.h[4]));
-            agt[a] = fd.adv;
-            kgt[a] = fd.ko;
-        }
+        for (int d = 0; d < 3; ++d) sc[3 * a + d] = fd.d[d];
+        // term 1: -1/2 gtu^{lm} d_l d_m gt_ij
+        sc[S_RT + a] = (P)-0.5 * (gtu[0] * fd.h[0] + gtu[3] * fd.h[3] + gtu[5] * fd.h[5] +
+                                        (P)2 * (gtu[1] * fd.h[1] + gtu[2] * fd.h[2] + gtu[4] * fd.h[4]));
+        sc[S_AG + a] = fd.adv;
+        if constexpr (EXACT) sc[S_KG + a] = fd.ko;
     }
+#pragma unroll
+    for (int a = 0; a < 6; ++a)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) dg[a][d] = sc[3 * a + d];
+    // the rest of the pointwise state, not needed by the loop above
+    const double alpha_d = __ldg(FP(ALPHA));
+    const P alpha = (P)alpha_d, K = (P)__ldg(FP(KTR)), Theta = (P)__ldg(FP(THETA));
+    P At[6], Gh[3];
+#pragma unroll
+    for (int a = 0; a < 6; ++a) At[a] = (P)__ldg(FP(AXX + a));
+#pragma unroll
+    for (int a = 0; a < 3; ++a) Gh[a] = (P)__ldg(FP(GHX + a));
+
     // first-kind Christoffels G1[k][ij] = 1/2 (d_i g_kj + d_j g_ki - d_k g_ij)
     P G1[3][6];
 #pragma unroll
@@ -199,19 +182,20 @@ __device__ __forceinline__ void ccz4_point(const DevBlock& B, const double* __re
 
     // ---- Gamma-hat: gradient (Ricci term 2), advection --------------------
     P dGh[3][3];
-    P aGh[3], kGh[3];
-#pragma unroll
+#pragma unroll U3
     for (int a = 0; a < 3; ++a) {
-        FieldDer<P> fd = S.template der<false, EXACT>(GHX + a, beta, w);
+        FieldDer<P> fd = S.template der<false, EXACT, false>(GHX + a, advec);
 #pragma unroll
-        for (int d = 0; d < 3; ++d) dGh[a][d] = fd.d[d];
-        aGh[a] = fd.adv;
-        kGh[a] = fd.ko;
+        for (int d = 0; d < 3; ++d) sm[3 * a + d] = fd.d[d];
+        sm[S_AGH + a] = fd.adv;
+        if constexpr (EXACT) sm[S_KGH + a] = fd.ko;
     }
-    if constexpr (Src::HS) {
 #pragma unroll
-        for (int a = 0; a < 6; ++a) Rt[a] = hs[(18 + a) * (Src::HS ? Src::NT : 1)];
-    }
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) dGh[a][d] = sm[3 * a + d];
+#pragma unroll
+    for (int a = 0; a < 6; ++a) Rt[a] = sc[S_RT + a];
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -245,7 +229,7 @@ __device__ __forceinline__ void ccz4_point(const DevBlock& B, const double* __re
     }
 
     // ---- chi: Ricci chi-part (ccz4.cpp:518-541) -----------------------------
-    FieldDer<P> fchi = S.template der<true, EXACT>(CHI, beta, w);
+    FieldDer<P> fchi = S.template der<true, EXACT, false>(CHI, advec);
     const P chiP = (P)chi;
     // 0.5/(chi+1e-30) and 0.25/(chi^2+1e-30) in FP64 (small chi near the puncture)
     const P c_half = (P)(0.5 / (chi + 1e-30));
@@ -279,7 +263,7 @@ __device__ __forceinline__ void ccz4_point(const DevBlock& B, const double* __re
     Rs *= chiP;
 
     // ---- lapse -------------------------------------------------------------
-    FieldDer<P> fal = S.template der<true, EXACT>(ALPHA, beta, w);
+    FieldDer<P> fal = S.template der<true, EXACT, false>(ALPHA, advec);
     P DDa[6];
 #pragma unroll
     for (int ij = 0; ij < 6; ++ij)
@@ -296,21 +280,27 @@ __device__ __forceinline__ void ccz4_point(const DevBlock& B, const double* __re
     // ---- shift: gradient, Hessian terms T5/T6 ---------------------------------
     P db[3][3];  // d_j beta^i as db[i][j]
     P T5[3], ddiv[3];
-    P abe[3], kbe[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) ddiv[d] = (P)0;
-#pragma unroll
+#pragma unroll U3
     for (int a = 0; a < 3; ++a) {
-        FieldDer<P> fb = S.template der<true, EXACT>(BETAX + a, beta, w);
+        FieldDer<P> fb = S.template der<true, EXACT, false>(BETAX + a, advec);
 #pragma unroll
-        for (int d = 0; d < 3; ++d) db[a][d] = fb.d[d];
-        T5[a] = gtu[0] * fb.h[0] + gtu[3] * fb.h[3] + gtu[5] * fb.h[5] +
+        for (int d = 0; d < 3; ++d) sm[3 * a + d] = fb.d[d];
+        sm[9 + a] = gtu[0] * fb.h[0] + gtu[3] * fb.h[3] + gtu[5] * fb.h[5] +
             (P)2 * (gtu[1] * fb.h[1] + gtu[2] * fb.h[2] + gtu[4] * fb.h[4]);
         // d_j (d_k beta^k): add d_j d_a beta^a
+        ddiv[0] += a == 0 ? fb.h[0] : (a == 1 ? fb.h[1] : fb.h[2]);
+        ddiv[1] += a == 0 ? fb.h[1] : (a == 1 ? fb.h[3] : fb.h[4]);
+        ddiv[2] += a == 0 ? fb.h[2] : (a == 1 ? fb.h[4] : fb.h[5]);
+        sm[S_AB + a] = fb.adv;
+        if constexpr (EXACT) sm[S_KB + a] = fb.ko;
+    }
 #pragma unroll
-        for (int d = 0; d < 3; ++d) ddiv[d] += fb.h[sy(a, d)];
-        abe[a] = fb.adv;
-        kbe[a] = fb.ko;
+    for (int a = 0; a < 3; ++a) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) db[a][d] = sm[3 * a + d];
+        T5[a] = sm[9 + a];
     }
     const P divb = db[0][0] + db[1][1] + db[2][2];  // :548
 
@@ -345,26 +335,19 @@ __device__ __forceinline__ void ccz4_point(const DevBlock& B, const double* __re
     // each field: (RHS incl. advection) + KO, the order of ccz4.cpp:864,930
     out[CHI] = (((P)(2.0 / 3.0) * chiP * (alpha * K - divb) + fchi.adv) + fchi.ko);
     // gt (ccz4.cpp:586-607)
-    if constexpr (Src::HS) {
-#pragma unroll
-        for (int a = 0; a < 6; ++a) {
-            agt[a] = hs[(24 + a) * (Src::HS ? Src::NT : 1)];
-            kgt[a] = hs[(30 + a) * (Src::HS ? Src::NT : 1)];
-        }
-    }
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
         for (int j = i; j < 3; ++j) {
             const int ij = sy(i, j);
-            P lie = agt[ij];
+            P lie = sc[S_AG + ij];
 #pragma unroll
             for (int d = 0; d < 3; ++d) lie += gt[sy(i, d)] * db[d][j] + gt[sy(j, d)] * db[d][i];
-            out[GXX + ij] = (((P)-2 * alpha * At[ij] + lie - (P)(2.0 / 3.0) * gt[ij] * divb) + kgt[ij]);
+            out[GXX + ij] = with_ko((P)-2 * alpha * At[ij] + lie - (P)(2.0 / 3.0) * gt[ij] * divb, S_KG + ij);
         }
     // K (ccz4.cpp:650-652)
     {
-        FieldDer<P> fK = S.template der<false, EXACT>(KTR, beta, w);
+        FieldDer<P> fK = S.template der<false, EXACT, false>(KTR, advec);
         const P k1 = (P)A.kappa1, k2 = (P)A.kappa2;
         out[KTR] = ((-phys_lap_alpha + alpha * (AtAt + K * K / (P)3) + (P)4 * PI * alpha * (rho + Str) +
                             k1 * ((P)1 - k2) * alpha * Theta + fK.adv) + fK.ko);
@@ -383,33 +366,37 @@ __device__ __forceinline__ void ccz4_point(const DevBlock& B, const double* __re
             const P T6 = (P)(1.0 / 3.0) *
                 (gtu[sy(i, 0)] * ddiv[0] + gtu[sy(i, 1)] * ddiv[1] + gtu[sy(i, 2)] * ddiv[2]);
             P T7 = -(Gh[0] * db[i][0] + Gh[1] * db[i][1] + Gh[2] * db[i][2]);
-            T7 += aGh[i] + (P)(2.0 / 3.0) * Gh[i] * divb;
+            T7 += sm[S_AGH + i] + (P)(2.0 / 3.0) * Gh[i] * divb;
             const P T8 = (P)-2 * (P)A.kappa1 * alpha * Gh[i];
-            out[GHX + i] = ((T1 + T2 + T3 + T4 + T5[i] + T6 + T7 + T8) + kGh[i]);
+            out[GHX + i] = with_ko(T1 + T2 + T3 + T4 + T5[i] + T6 + T7 + T8, S_KGH + i);
         }
+    }
+    // Theta and A-tilde: only advection and KO (slots 0-6 and 7-13)
+#pragma unroll U7
+    for (int p = 0; p < 7; ++p) {
+        FieldDer<P> fd = S.template der<false, EXACT, true>(FIELD_ORDER[15 + p], advec);
+        sm[p] = fd.adv;
+        sm[7 + p] = fd.ko;
     }
     // Theta (ccz4.cpp:662-665)
     {
-        FieldDer<P> fT = S.template der<false, EXACT>(THETA, beta, w);
         const P k1 = (P)A.kappa1, k2 = (P)A.kappa2;
         out[THETA] = (((P)0.5 * alpha * (Rs - AtAt + (P)2 * K * K / (P)3 - (P)16 * PI * rho) -
-                              alpha * k1 * ((P)2 + k2) * Theta + fT.adv) + fT.ko);
+                              alpha * k1 * ((P)2 + k2) * Theta + sm[0]) + sm[7]);
     }
     // A-tilde (ccz4.cpp:671-726): the advection is part of Lie_At and is
     // trace-removed with the rest; KO is added after the trace removal.
     {
-        P raw[6], koA[6];
+        P raw[6];
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
             for (int j = i; j < 3; ++j) {
                 const int ij = sy(i, j);
-                FieldDer<P> fA = S.template der<false, EXACT>(AXX + ij, beta, w);
-                koA[ij] = fA.ko;
                 const P t1 = chiP * (-DDa[ij] + alpha * (Ric[ij] - (P)8 * PI * Sij[ij]));
                 const P Asq = At[sy(i, 0)] * Am[0][j] + At[sy(i, 1)] * Am[1][j] + At[sy(i, 2)] * Am[2][j];
                 const P t2 = alpha * (K * At[ij] - (P)2 * Asq);
-                P lie = fA.adv;
+                P lie = sm[1 + ij];
 #pragma unroll
                 for (int d = 0; d < 3; ++d) lie += At[sy(i, d)] * db[d][j] + At[sy(j, d)] * db[d][i];
                 lie -= (P)(2.0 / 3.0) * At[ij] * divb;
@@ -418,14 +405,14 @@ __device__ __forceinline__ void ccz4_point(const DevBlock& B, const double* __re
         const P tr = gtu[0] * raw[0] + gtu[3] * raw[3] + gtu[5] * raw[5] +
             (P)2 * (gtu[1] * raw[1] + gtu[2] * raw[2] + gtu[4] * raw[4]);
 #pragma unroll
-        for (int a = 0; a < 6; ++a) out[AXX + a] = (raw[a] - (P)(1.0 / 3.0) * gt[a] * tr + koA[a]);
+        for (int a = 0; a < 6; ++a) out[AXX + a] = (raw[a] - (P)(1.0 / 3.0) * gt[a] * tr + sm[8 + a]);
     }
     // lapse (ccz4.cpp:820) and shift (ccz4.cpp:825-831)
     out[ALPHA] = (((P)-2 * alpha * K + fal.adv) + fal.ko);
     {
         const P eta = (P)A.eta;
 #pragma unroll
-        for (int d = 0; d < 3; ++d) out[BETAX + d] = (((P)0.75 * Gh[d] - eta * (P)beta[d] + abe[d]) + kbe[d]);
+        for (int d = 0; d < 3; ++d) out[BETAX + d] = with_ko((P)0.75 * Gh[d] - eta * bp[d] + sm[S_AB + d], S_KB + d);
     }
 #undef FP
 }
@@ -492,9 +479,6 @@ __device__ __forceinline__ void point_pm(const DevBlock& B, const double* __rest
 }
 
 // Shared epilogue: store L, or RK combine + floors (+ algebraic constraints).
-// u_in: the stage input at the point, from global memory, or (tin != nullptr)
-// from a per-thread column of shared memory that the stencil source filled with
-// each field's centre value, field v at tin[v * tin_stride].
 // The new state of interior point (i, j, k) into the ghost cells of the
 // same-level neighbours that hold it (the tile's npush boxes, slot out_sel);
 // the containment test is per point.
@@ -513,7 +497,6 @@ __device__ __forceinline__ void push_copies(const PushBox* boxes, int npush, int
 // interior indices, for the pushed ghost copies.
 template <int EPI, typename T>
 __device__ __forceinline__ void stage_epilogue(const DevBlock& B, const StageArgs& A, long long c, const T L[NV],
-                                               const double* tin = nullptr, int tin_stride = 0,
                                                const PushBox* pushes = nullptr, int npush = 0, int i = 0, int j = 0,
                                                int k = 0) {
     const long long st = B.stride;
@@ -526,19 +509,7 @@ __device__ __forceinline__ void stage_epilogue(const DevBlock& B, const StageArg
     const double* __restrict__ un = B.buf[A.n_sel];
     double* __restrict__ out = B.buf[A.out_sel];
     double r[NV];
-    if (tin) {
-        if (A.in_sel == A.n_sel) {
-#pragma unroll
-            for (int v = 0; v < NV; ++v) {
-                const double unv = tin[v * tin_stride];
-                r[v] = rk_combine(A.a1, unv, A.a2, unv, A.a3dt, L[v]);
-            }
-        } else {
-#pragma unroll
-            for (int v = 0; v < NV; ++v)
-                r[v] = rk_combine(A.a1, __ldg(un + (long long)v * st + c), A.a2, tin[v * tin_stride], A.a3dt, L[v]);
-        }
-    } else if (A.in_sel == A.n_sel) {  // stage 1 reads u^n as both the stage input and u^n: load it once
+    if (A.in_sel == A.n_sel) {  // stage 1 reads u^n as both the stage input and u^n: load it once
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
             const double unv = __ldg(un + (long long)v * st + c);

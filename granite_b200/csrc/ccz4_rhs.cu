@@ -6,7 +6,7 @@
 // a work-list of tiles over every block of an AMR level, so blocks of uneven
 // size share one launch per RK stage. The per-point body is ccz4_point
 // (ccz4_point.cuh); the TMA-ring variant is in ccz4_stage_tma.cuh, instantiated
-// per tuning configuration in ccz4_tma_cfg<k>.cu.
+// per tile set in ccz4_tma_tiles<k>.cu.
 //
 // Per-tile precision: a launch can be restricted to the tiles of a flag array
 // (classify_tiles_kernel marks the tiles with a point of chi below a threshold,
@@ -87,7 +87,7 @@ struct TileGeom {
 // every field in order (the calls carry the CTA barrier).
 template <int TX, int TY, int TZ, int NBUF>
 struct SmemSource {
-    static constexpr bool HS = false, UNROLL = false;
+    static constexpr bool UNROLL = true;
     using G = TileGeom<TX, TY, TZ>;
     const DevBlock& B;
     const double* __restrict__ u;  // stencil buffer (global)
@@ -111,15 +111,15 @@ struct SmemSource {
     __device__ __forceinline__ void start() {
         for (int k = 0; k < NBUF - 1; ++k) issue(k);
     }
-    template <bool HESS, bool EXACT, typename P>
-    __device__ __forceinline__ FieldDer<P> der(int /*v*/, const double beta[3], P w) {
+    __device__ __forceinline__ const StencilCoef& coefs() const { return B; }
+    template <bool HESS, bool EXACT, bool KOSEP, typename P>
+    __device__ __forceinline__ FieldDer<P> der(int /*v*/, const Advection<P, EXACT>& adv) {
         cp_async_wait<NBUF - 2>();
         __syncthreads();
         issue(next + NBUF - 1);
-        const long long off[3] = {1, G::BX, G::BX * G::BY};
-        const SharedLoad L{sm + (next % NBUF) * G::BOX + lin};
+        const SharedLoad<G::BX, G::BX * G::BY> L{sm + (next % NBUF) * G::BOX + lin};
         ++next;
-        return field_der_l<P, HESS, true, SharedLoad, EXACT>(B, L, off, beta, w);
+        return field_der_l<P, HESS, true, EXACT, KOSEP>(B, L, adv);
     }
 };
 
@@ -221,13 +221,12 @@ __global__ void __launch_bounds__(32 * CLASSIFY_WARPS)
 constexpr int V0_TX = 32, V0_TY = 4, V0_TZ = 1;
 constexpr int V1_TX = 16, V1_TY = 4, V1_TZ = 2, V1_NBUF = 3;
 
-int stage_tile_dims(int variant, int cfg, int* tx, int* ty, int* tz) {
+void stage_tile_dims(int variant, int* tx, int* ty, int* tz) {
     if (variant == VARIANT_TMA) {
-        if (cfg < 0 || cfg >= NUM_TMA_CFGS) return -1;
         *tx = 16;
         *ty = 4;
-        *tz = TMA_CFGS[cfg].tz;
-    } else if (variant == 1) {
+        *tz = TMA_TZ;
+    } else if (variant == VARIANT_SMEM) {
         *tx = V1_TX;
         *ty = V1_TY;
         *tz = V1_TZ;
@@ -236,7 +235,6 @@ int stage_tile_dims(int variant, int cfg, int* tx, int* ty, int* tz) {
         *ty = V0_TY;
         *tz = V0_TZ;
     }
-    return 0;
 }
 
 template <int PM, int EPI>
@@ -257,88 +255,33 @@ static cudaError_t configure_smem() {
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
-// The TMA configurations, one translation unit each (ccz4_tma_cfg<k>.cu).
+// The tile sets of the TMA kernel, one translation unit each (ccz4_tma_tiles<k>.cu).
 using TmaConfigure = cudaError_t (*)(int nsm, int grids[3][2][2]);
 using TmaLaunch = cudaError_t (*)(int pm, int epi, bool sel, const DevBlock* blocks, const Tile* tiles, int ntiles,
                                   const StageArgs& args, cudaStream_t stream, int grid);
-cudaError_t configure_tma_cfg0(int, int[3][2][2]);
-cudaError_t configure_tma_cfg1(int, int[3][2][2]);
-cudaError_t configure_tma_cfg2(int, int[3][2][2]);
-cudaError_t configure_tma_cfg3(int, int[3][2][2]);
-cudaError_t configure_tma_cfg4(int, int[3][2][2]);
-cudaError_t configure_tma_cfg5(int, int[3][2][2]);
-cudaError_t configure_tma_cfg6(int, int[3][2][2]);
-cudaError_t configure_tma_cfg7(int, int[3][2][2]);
-cudaError_t configure_tma_cfg8(int, int[3][2][2]);
-cudaError_t configure_tma_cfg9(int, int[3][2][2]);
-cudaError_t configure_tma_cfg10(int, int[3][2][2]);
-cudaError_t configure_tma_cfg11(int, int[3][2][2]);
-cudaError_t configure_tma_cfg12(int, int[3][2][2]);
-cudaError_t configure_tma_cfg13(int, int[3][2][2]);
-cudaError_t configure_tma_cfg14(int, int[3][2][2]);
-cudaError_t configure_tma_cfg15(int, int[3][2][2]);
-cudaError_t configure_tma_cfg16(int, int[3][2][2]);
-cudaError_t configure_tma_cfg17(int, int[3][2][2]);
-cudaError_t launch_tma_cfg0(int, int, bool, const DevBlock*, const Tile*, int, const StageArgs&, cudaStream_t, int);
-cudaError_t launch_tma_cfg1(int, int, bool, const DevBlock*, const Tile*, int, const StageArgs&, cudaStream_t, int);
-cudaError_t launch_tma_cfg2(int, int, bool, const DevBlock*, const Tile*, int, const StageArgs&, cudaStream_t, int);
-cudaError_t launch_tma_cfg3(int, int, bool, const DevBlock*, const Tile*, int, const StageArgs&, cudaStream_t, int);
-cudaError_t launch_tma_cfg4(int, int, bool, const DevBlock*, const Tile*, int, const StageArgs&, cudaStream_t, int);
-cudaError_t launch_tma_cfg5(int, int, bool, const DevBlock*, const Tile*, int, const StageArgs&, cudaStream_t, int);
-cudaError_t launch_tma_cfg6(int, int, bool, const DevBlock*, const Tile*, int, const StageArgs&, cudaStream_t, int);
-cudaError_t launch_tma_cfg7(int, int, bool, const DevBlock*, const Tile*, int, const StageArgs&, cudaStream_t, int);
-cudaError_t launch_tma_cfg8(int, int, bool, const DevBlock*, const Tile*, int, const StageArgs&, cudaStream_t, int);
-cudaError_t launch_tma_cfg9(int, int, bool, const DevBlock*, const Tile*, int, const StageArgs&, cudaStream_t, int);
-cudaError_t launch_tma_cfg10(int, int, bool, const DevBlock*, const Tile*, int, const StageArgs&, cudaStream_t, int);
-cudaError_t launch_tma_cfg11(int, int, bool, const DevBlock*, const Tile*, int, const StageArgs&, cudaStream_t, int);
-cudaError_t launch_tma_cfg12(int, int, bool, const DevBlock*, const Tile*, int, const StageArgs&, cudaStream_t, int);
-cudaError_t launch_tma_cfg13(int, int, bool, const DevBlock*, const Tile*, int, const StageArgs&, cudaStream_t, int);
-cudaError_t launch_tma_cfg14(int, int, bool, const DevBlock*, const Tile*, int, const StageArgs&, cudaStream_t, int);
-cudaError_t launch_tma_cfg15(int, int, bool, const DevBlock*, const Tile*, int, const StageArgs&, cudaStream_t, int);
-cudaError_t launch_tma_cfg16(int, int, bool, const DevBlock*, const Tile*, int, const StageArgs&, cudaStream_t, int);
-cudaError_t launch_tma_cfg17(int, int, bool, const DevBlock*, const Tile*, int, const StageArgs&, cudaStream_t, int);
-static_assert(NUM_TMA_CFGS == 18, "one configure / launch pair per TMA configuration");
-static const TmaConfigure g_tma_configure[NUM_TMA_CFGS] = {
-    configure_tma_cfg0, configure_tma_cfg1, configure_tma_cfg2, configure_tma_cfg3, configure_tma_cfg4, configure_tma_cfg5,
-    configure_tma_cfg6, configure_tma_cfg7, configure_tma_cfg8, configure_tma_cfg9, configure_tma_cfg10,
-    configure_tma_cfg11, configure_tma_cfg12, configure_tma_cfg13, configure_tma_cfg14, configure_tma_cfg15,
-    configure_tma_cfg16, configure_tma_cfg17};
-static const TmaLaunch g_tma_launch[NUM_TMA_CFGS] = {
-    launch_tma_cfg0, launch_tma_cfg1, launch_tma_cfg2, launch_tma_cfg3, launch_tma_cfg4, launch_tma_cfg5,
-    launch_tma_cfg6, launch_tma_cfg7, launch_tma_cfg8, launch_tma_cfg9, launch_tma_cfg10, launch_tma_cfg11,
-    launch_tma_cfg12, launch_tma_cfg13, launch_tma_cfg14, launch_tma_cfg15, launch_tma_cfg16, launch_tma_cfg17};
+cudaError_t configure_tma_tiles0(int, int[3][2][2]);
+cudaError_t configure_tma_tiles1(int, int[3][2][2]);
+cudaError_t launch_tma_tiles0(int, int, bool, const DevBlock*, const Tile*, int, const StageArgs&, cudaStream_t, int);
+cudaError_t launch_tma_tiles1(int, int, bool, const DevBlock*, const Tile*, int, const StageArgs&, cudaStream_t, int);
+static const TmaConfigure g_tma_configure[NUM_TMA_TILESETS] = {configure_tma_tiles0, configure_tma_tiles1};
+static const TmaLaunch g_tma_launch[NUM_TMA_TILESETS] = {launch_tma_tiles0, launch_tma_tiles1};
 
-// Persistent grid of each TMA configuration on each device: SMs x resident CTAs.
+// Persistent grid of each TMA kernel on each device (one CTA per SM).
 constexpr int MAX_DEVICES = 64;
-static int g_tma_grid[MAX_DEVICES][NUM_TMA_CFGS][3][2][2];  // [device][cfg][precision mode][epi][sel]
+static int g_tma_grid[MAX_DEVICES][NUM_TMA_TILESETS][3][2][2];  // [device][tile set][precision mode][epi][sel]
 
-int tma_grid(int cfg) {
-    int dev = 0;
-    if (cfg < 0 || cfg >= NUM_TMA_CFGS) return 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return 0;
-    // the smaller of the two per-tile passes' resident grids (the FP64 pass may
-    // fit fewer CTAs per SM)
-    const int a = g_tma_grid[dev][cfg][PM_MIXED][EPI_RK][1], b = g_tma_grid[dev][cfg][PM_FP64F][EPI_RK][1];
-    return a < b ? a : b;
-}
-
-static cudaError_t launch_tma(int cfg, int pm, int epi, const DevBlock* blocks, const Tile* tiles, int ntiles,
+static cudaError_t launch_tma(int tileset, int pm, int epi, const DevBlock* blocks, const Tile* tiles, int ntiles,
                               const StageArgs& args, cudaStream_t stream) {
-    if (!args.tmaps || cfg < 0 || cfg >= NUM_TMA_CFGS || pm < 0 || pm > 2) return cudaErrorInvalidValue;
-    if (TMA_CFGS[cfg].rem && !args.tmaps_rem) return cudaErrorInvalidValue;
+    if (!args.tmaps || tileset < 0 || tileset >= NUM_TMA_TILESETS || pm < 0 || pm > 2) return cudaErrorInvalidValue;
+    if (!args.tmaps_arm || (tileset == 1 && !args.tmaps_rem)) return cudaErrorInvalidValue;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     const bool sel = args.tile_prec != nullptr;  // per-tile precision passes (RK epilogue)
     if (sel && epi != EPI_RK) return cudaErrorInvalidValue;
-    int cap = (dev >= 0 && dev < MAX_DEVICES) ? g_tma_grid[dev][cfg][pm][epi][sel ? 1 : 0] : 0;
+    const int cap = (dev >= 0 && dev < MAX_DEVICES) ? g_tma_grid[dev][tileset][pm][epi][sel ? 1 : 0] : 0;
     if (cap <= 0) return cudaErrorInvalidConfiguration;  // not instantiated, or configure_stage_kernels() not run
-    // The FP64 pass of the per-tile precision takes few tiles, clustered near the
-    // punctures: TMA_FP64_SPREAD times the resident grid spreads them over more
-    // CTAs (a CTA without selected tiles exits after its scan), so fewer CTAs run
-    // two or more of them one after the other.
-    if (pm == PM_FP64F && sel) cap *= TMA_FP64_SPREAD;
-    return g_tma_launch[cfg](pm, epi, sel, blocks, tiles, ntiles, args, stream, ntiles < cap ? ntiles : cap);
+    return g_tma_launch[tileset](pm, epi, sel, blocks, tiles, ntiles, args, stream, ntiles < cap ? ntiles : cap);
 }
 
 // Opt the shared-memory variants into more than 48 KB of dynamic shared memory
@@ -355,7 +298,7 @@ cudaError_t configure_stage_kernels() {
     if ((e = cudaGetDevice(&dev))) return e;
     if (dev < 0 || dev >= MAX_DEVICES) return cudaErrorInvalidDevice;
     if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev))) return e;
-    for (int k = 0; k < NUM_TMA_CFGS; ++k)
+    for (int k = 0; k < NUM_TMA_TILESETS; ++k)
         if ((e = g_tma_configure[k](nsm, g_tma_grid[dev][k]))) return e;
     return cudaSuccess;
 }
@@ -398,21 +341,21 @@ struct RunGlobal {
     };
 };
 
-cudaError_t launch_classify(int variant, int cfg, const DevBlock* blocks, const Tile* tiles, int first, int ntiles,
+cudaError_t launch_classify(int variant, const DevBlock* blocks, const Tile* tiles, int first, int ntiles,
                             int sel, double chi_fp64, unsigned char* flag, cudaStream_t stream) {
     if (ntiles <= 0) return cudaSuccess;
     int tx, ty, tz;
-    if (stage_tile_dims(variant, cfg, &tx, &ty, &tz)) return cudaErrorInvalidValue;
+    stage_tile_dims(variant, &tx, &ty, &tz);
     classify_tiles_kernel<<<(ntiles + CLASSIFY_WARPS - 1) / CLASSIFY_WARPS, 32 * CLASSIFY_WARPS, 0, stream>>>(
         blocks, tiles, first, ntiles, sel, tx, ty, tz, chi_fp64, flag);
     return cudaGetLastError();
 }
 
-cudaError_t launch_stage(int variant, int cfg, int precision, int epi, const DevBlock* blocks, const Tile* tiles,
+cudaError_t launch_stage(int variant, int tileset, int precision, int epi, const DevBlock* blocks, const Tile* tiles,
                          int ntiles, const StageArgs& args, cudaStream_t stream) {
     if (ntiles <= 0) return cudaSuccess;
     switch (variant) {
-        case VARIANT_TMA: return launch_tma(cfg, precision, epi, blocks, tiles, ntiles, args, stream);
+        case VARIANT_TMA: return launch_tma(tileset, precision, epi, blocks, tiles, ntiles, args, stream);
         case VARIANT_SMEM: return dispatch<RunSmem>(precision, epi, blocks, tiles, ntiles, args, stream);
         case VARIANT_GLOBAL_R168:
             return dispatch<RunGlobal<3>::L>(precision, epi, blocks, tiles, ntiles, args, stream);

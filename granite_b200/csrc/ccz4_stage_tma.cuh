@@ -1,33 +1,43 @@
-// ccz4_stage_tma.cuh -- the TMA-ring stage kernel, templated on its tuning
-// configuration. Each ccz4_tma_cfg<k>.cu instantiates one entry of TMA_CFGS
-// (ccz4_kernels.h), so the configurations compile in parallel and the
-// autotuner can pick one per block-size class at run time.
+// ccz4_stage_tma.cuh -- the TMA stage kernel.
 //
-// A persistent CTA walks its tiles (blockIdx.x, + gridDim.x, ...) and consumes
-// a stream of items q = (tile round q / NV, field FIELD_ORDER[q % NV]). Item q
-// is one (16 + 8) x (4 + 8) x (TZ + 8)-cell box (the 16 x 4 x TZ tile and its
-// 4-cell halo) of one field, brought into ring slot q % NBUF by a single
-// cp.async.bulk.tensor load that completes on that slot's mbarrier. Every BAR
-// items (BAR = 1 or 2) the CTA meets at a barrier, after which the slots of
-// the last BAR items are free and thread 0 issues items q + NBUF - BAR ..
-// q + NBUF - 1 into them: loads run NBUF - BAR to NBUF - 1 fields ahead, across
-// tile boundaries. Rows of 24 doubles put the 16-wide x rows of a warp in
-// distinct shared-memory banks for every stencil offset.
+// One CTA per SM: NWG compute warpgroups (128 threads, one 16 x 4 x 2 tile
+// each) and one warpgroup of load warps, load warp g serving compute
+// warpgroup g. Each pair is independent of the others: it walks its own tiles
+// (CTA b's warpgroup g: list entries g gridDim.x + b, + gridDim.x NWG, ...) through
+// its own ring of field boxes.
 //
-// Options of a configuration:
-//   TIN  every field's centre value is copied from the ring into a per-thread
-//        column of shared memory as it streams through, and the RK epilogue
-//        reads the stage input there instead of from global memory;
-//   PF   the epilogue's u^n cells and the next tile's pointwise cells are
-//        prefetched into L2 at the start of each tile (always with TIN);
-//   HS   the 36 values of the Hessian-field loop live in a per-thread column of
-//        shared memory instead of local memory;
-//   MINB resident CTAs per SM that the register allocation is sized for
-//        (__launch_bounds__): 3 CTAs of 128 threads cap a thread at 168
-//        registers, and the ring (with or without TIN) still fits three times in
-//        an SM's shared memory;
-//   BAR  ring items per CTA barrier: 2 halves the barriers of a tile (22 fields)
-//        at the price of a shallower look-ahead on every other item.
+//   load warp:   finds the next tile (with per-tile precision the next one whose
+//                flag the launch takes, a ballot over 32 flags at a time),
+//                copies it and its block's descriptor into shared memory one round
+//                ahead, and per field waits until the slot is empty and issues
+//                the field's three box loads (TileBoxes);
+//   compute warps: per field wait for the slot's boxes, evaluate the stencils,
+//                arrive on the slot's empty barrier (one arrival per warp) and
+//                go on; no barrier among the warps. The algebra is ccz4_point.
+//
+// What bounds it: instruction issue (67 % of the slots) and latency at 12 compute
+// warps per SM in the mixed form, latency at 8 in the FP64 form. What measured
+// (128 x 128 x 64 points, stage 1-3 average, mixed / FP64): 508 / 685 us when two
+// CTAs of 128 threads (one of 256) issued their own loads, one 24 x 12 x (tz + 8)
+// box per field behind a CTA barrier, with generic loads of the ring and the
+// stencil coefficients in global memory; 424 / 523 with shared-space loads,
+// coefficients in the kernel arguments and tiles and descriptors copied ahead;
+// 343 / 470 with the load warps, three boxes per field, rolled field loops and
+// 32-bit shared addresses. Per field a barrier cost a fifth of the stall cycles
+// (a third with three boxes to issue). Prefetching the next tile's fields into
+// L2 from the load warps: 20 % slower (the burst delays the ring's own loads).
+// Ring slots per mixed warpgroup 3 / 4 / 5: 343 / 351 / 375 (they take L1 from the
+// per-point body's local memory).
+//
+// Registers: the launch gives every thread 65536 / threads; setmaxnreg moves
+// the load warpgroup's to the compute warpgroups (the shares below add up to at
+// most the launch's total, which TmaKernelOps checks).
+//
+// Every wait is bounded (TMA_WAIT_NS): a thread whose wait gives up records it
+// in StageArgs::errflag and skips its later waits; a compute warp then leaves
+// after its current tile, and a load warp stops issuing, waits (bounded) for
+// the copies it issued and leaves, so the kernel always ends and no copy into
+// shared memory outlives the CTA.
 #pragma once
 
 #include <cstdint>
@@ -39,40 +49,26 @@ namespace granite_b200 {
 
 namespace {
 
-template <int TZ_, int NBUF_, bool TIN_, bool HS_, int MINB_, int BAR_ = 1, int REM_ = 0, bool PF_ = false>
-struct TmaCfgT {
-    static constexpr int TZ = TZ_, NBUF = NBUF_, BAR = BAR_;
-    // a tile round's first item starts a barrier group (the round's shared push
-    // boxes rely on it), and at least one item is loaded ahead
-    static_assert((BAR == 1 || BAR == 2) && NV % BAR == 0 && NBUF > BAR, "barrier grouping");
-    static constexpr bool TIN = TIN_, HS = HS_;
-    // x-remainder tiles: REM, one box of the 2 TZ shape per field; REM2, two
-    // boxes of this configuration's own shape per field (one per half of the
-    // tile along z), two ring items that one barrier group frees together
-    static constexpr bool REM = REM_ == 1, REM2 = REM_ == 2;
-    static constexpr bool PF = TIN || PF_;  // the L2 prefetches at the start of each tile
-    static constexpr int TX = 16, TY = 4, NT = TX * TY * TZ;
-    static_assert(!REM2 || (BAR == 2 && TMA_REM_X * TY * 2 * TZ == NT), "two-box remainder tiles");
-    static constexpr int MINB = MINB_;  // resident CTAs per SM asked of the register allocator
-    static constexpr int BX = TX + 8, BY = TY + 8, BZ = TZ + 8;
-    static constexpr int BOX = BX * BY * BZ;
-    static constexpr unsigned BYTES = BOX * sizeof(double);  // complete_tx count of one item
-    // x-remainder tiles: TMA_REM_X x TY x 2 TZ points, the same rows (BX, BY) and
-    // 2 TZ + 8 planes per box, so the stencil offsets stay those of the full tiles
-    static_assert(!REM || (tma_shape_for_tz(2 * TZ) >= 0 && TMA_REM_X * TY * 2 * TZ == NT),
-                  "remainder tiles: one point per thread, loaded with the 2 TZ box shape");
-    static constexpr int BOX_REM = BX * BY * (2 * TZ + 8);
-    static constexpr unsigned BYTES_REM = BOX_REM * sizeof(double);
-    static constexpr int SLOT = REM ? BOX_REM : BOX;  // doubles per ring slot
-    static_assert(BYTES % 128 == 0 && (SLOT * sizeof(double)) % 128 == 0, "slots stay 128-byte aligned");
-    static_assert(BX == TMA_BOX_X && BY == TMA_BOX_Y, "box = tile + halo");
-    // dynamic shared memory: ring | mbarriers | stage-input column | Hessian slots
-    static constexpr size_t OFF_BAR = (size_t)NBUF * SLOT * sizeof(double);
-    static constexpr size_t OFF_TIN = (OFF_BAR + NBUF * sizeof(unsigned long long) + 127) / 128 * 128;
-    static constexpr size_t OFF_HS = OFF_TIN + (TIN ? (size_t)NV * NT * sizeof(double) : 0);
-    template <typename P>
-    static constexpr size_t smem() {
-        return OFF_HS + (HS ? (size_t)36 * NT * sizeof(P) : 0) + 128;  // + alignment of the base
+// The boxes of one field of a tile of depth TZ in a ring slot (ccz4_kernels.h):
+// the main box, then the far planes below and above it.
+template <int TZ>
+struct TileBoxes {
+    static constexpr int BX = TMA_BOX_X, BY = TMA_BOX_Y;
+    static constexpr int MAIN = BX * BY * (TZ + 2), ARM = TMA_ARM_X * TMA_ARM_Y * TMA_ARM_Z;
+    static constexpr int CELLS = MAIN + 2 * ARM;
+    static_assert(MAIN * sizeof(double) % 128 == 0 && ARM * sizeof(double) % 128 == 0, "boxes stay 128-byte aligned");
+    // offset of tile point (x, y, z)
+    static __device__ __forceinline__ int point(int x, int y, int z) { return (x + 4) + BX * ((y + 4) + BY * (z + 1)); }
+    static __device__ __forceinline__ int plane(int x, int y, int z) {
+        const int a = x + TMA_ARM_X * y, p = TMA_ARM_X * TMA_ARM_Y;
+        return z < -1 ? MAIN + a + p * (z + 4) : (z > TZ ? MAIN + ARM + a + p * (z - TZ - 1) : point(x, y, z));
+    }
+    static __device__ __forceinline__ void arms(int x, int y, int z, ArmOffsets& o) {
+#pragma unroll
+        for (int k = 2; k <= 4; ++k) {
+            o.lo[k - 2] = plane(x, y, z - k) * (int)sizeof(double);
+            o.hi[k - 2] = plane(x, y, z + k) * (int)sizeof(double);
+        }
     }
 };
 
@@ -93,18 +89,6 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity) {
         : "memory");
     return ok != 0;
 }
-// The same test with a suspend-time hint: a thread whose phase is not complete
-// yet is suspended (issuing nothing) until it completes or about hint_ns pass,
-// instead of spinning.
-__device__ __forceinline__ bool mbar_try_wait_sleep(unsigned bar, unsigned parity, unsigned hint_ns) {
-    unsigned ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity), "r"(hint_ns)
-        : "memory");
-    return ok != 0;
-}
 __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -119,346 +103,339 @@ __device__ __forceinline__ void tma_load_box(unsigned dst, const void* map, int 
         "l"(map), "r"(x), "r"(y), "r"(z), "r"(f), "r"(bar)
         : "memory");
 }
-// Bring the line holding p into L2 with the evict-last priority (a hint: no
-// register, no completion to wait for).
-__device__ __forceinline__ void prefetch_l2(const double* p) {
-    asm volatile("prefetch.global.L2::evict_last [%0];" ::"l"(p));
-}
-
 // Wait limit of one ring slot: 2 s of wall time, then the kernel records the
 // failure in StageArgs::errflag and stops waiting (results are then garbage
 // and the host reports the error).
 constexpr unsigned long long TMA_WAIT_NS = 2000000000ull;
-// Suspend-time hint of one wait attempt (the limit is checked between attempts).
-constexpr unsigned TMA_WAIT_HINT_NS = 100000u;
+// NWG compute warpgroups, NBUF ring slots each; REM: x-remainder tiles
+// (TMA_REM_X x 4 x 4 points, slots sized for their boxes).
+template <int NWG_, int NBUF_, bool REM_>
+struct TmaKernelT {
+    static constexpr int NWG = NWG_, NBUF = NBUF_;
+    static constexpr bool REM = REM_;
+    static constexpr int TX = 16, TY = 4, TZ = 2, NP = TX * TY * TZ;
+    static constexpr int NTHR = (NWG + 1) * NP;
+    static constexpr int BX = TMA_BOX_X, BY = TMA_BOX_Y;
+    using Boxes = TileBoxes<TZ>;
+    using BoxesRem = TileBoxes<2 * TZ>;
+    static_assert(NP == 128 && NWG <= 4 && NBUF <= 4, "one load warp per compute warpgroup");
+    static_assert(TMA_REM_X * TY * 2 * TZ == NP, "remainder tiles: one point per thread");
+    static constexpr int SLOT = REM ? BoxesRem::CELLS : Boxes::CELLS;
+    static constexpr size_t SMEM = (size_t)NWG * NBUF * SLOT * sizeof(double);
+    // registers per thread: of the launch, of the load warps, of the compute warps
+    static constexpr int LAUNCH_REGS = 65536 / NTHR / 8 * 8;
+    static constexpr int LOAD_REGS = 40;  // (24 and 32 spill in the load warps: 8 % slower)
+    static constexpr int COMP_REGS = (LAUNCH_REGS * NTHR - LOAD_REGS * NP) / (NWG * NP) / 8 * 8;
+    static_assert(NWG * NP * COMP_REGS + NP * LOAD_REGS <= NTHR * LAUNCH_REGS, "the split moves registers, it adds none");
+    static_assert(COMP_REGS <= 255 && COMP_REGS >= 128, "compute warps");
+};
 
-// Per-tile precision launches: the CTA's selected tiles, in order, and their
-// count at [TMA_SEL_CAP] (shared memory at a fixed address, so the per-point
-// body keeps no register for them).
-__shared__ int g_sel_list[TMA_SEL_CAP + 1];
-
-template <class C, bool SEL>
-struct TmaSource {
-    static constexpr bool HS = C::HS, UNROLL = false;
-    static constexpr int NT = C::NT;
-    const DevBlock* blocks;
-    const Tile* tiles;
-    const unsigned char* maps;  // CUtensorMap array of this box shape, 128 bytes each
-    const unsigned char* maps_rem;  // REM: the same for the remainder tiles' box shape
-    int ntiles, in_sel;
-    double* ring;      // NBUF slots of C::SLOT doubles
-    unsigned bar0;     // shared address of the slot mbarriers (8 bytes apart)
-    double* tin;       // TIN: this thread's stage-input column (field v at tin[v * NT])
-    void* hs;          // HS: this thread's Hessian-loop column (slot q at hs[q * NT])
-    const DevBlock* B; // block of the current tile (stencil coefficients)
-    int lin;           // this thread's point within a slot
-    int next;          // next item to consume
-    bool failed;       // a wait of this thread gave up (at item fail_q); thread 0 then stops issuing
-    unsigned int* err;
-    int fail_q;
-    int withhold;      // test switch: 1 + the item CTA 0 leaves unissued (0: none)
-    // REM2: the item stream has 2 NV items in a remainder tile's round (field
-    // FIELD_ORDER[p / 2], half p % 2), NV in the others; thread 0 keeps its issue
-    // position as a cursor (round, position, items issued)
-    int ic_round = 0, ic_pos = 0, issued = 0;
-    bool rem_round = false;  // REM2: the current round is a remainder tile
-    int half = 0;            // REM2: this thread's half of a remainder tile
-
-    template <typename P>
-    __device__ __forceinline__ P* hess_slots() const {
-        return static_cast<P*>(hs);
-    }
-    // Tile of the CTA's r-th round: blockIdx.x + r gridDim.x, or with per-tile
-    // precision (SEL) the r-th tile of that sequence whose flag the launch takes.
-    __device__ __forceinline__ int round_tile(int r) const {
-        if constexpr (SEL)
-            return r < g_sel_list[TMA_SEL_CAP] ? g_sel_list[r] : ntiles;
-        else
-            return blockIdx.x + r * gridDim.x;
-    }
-    // thread 0 only
-    __device__ __forceinline__ void issue(int q) const {
-        const int ti = round_tile(q / NV);
-        if (ti >= ntiles) return;
-        if (withhold != 0 && q == withhold - 1 && blockIdx.x == 0) return;  // test switch: never issued
-        const Tile t = tiles[ti];
-        const bool rem = C::REM && t.w < 0;
-        const int s = q % C::NBUF;
-        const unsigned bar = bar0 + 8u * s;
-        mbar_expect_tx(bar, rem ? C::BYTES_REM : C::BYTES);
-        // box origin = tile origin - 4 cells = interior index (cells incl. ghosts start 4 lower)
-        tma_load_box(smem_addr(ring + (size_t)s * C::SLOT), (rem ? maps_rem : maps) + (size_t)(3 * t.block + in_sel) * 128,
-                     t.i0, t.j0, t.k0, FIELD_ORDER[q % NV], bar);
-    }
-    // thread 0 only (REM2): issue the next item of the stream
-    __device__ __forceinline__ void issue_next() {
-        const int ti = round_tile(ic_round);
-        if (ti >= ntiles) return;  // nothing after the CTA's last tile
-        const Tile t = tiles[ti];
-        const bool rem = t.w < 0;
-        const int q = issued++;
-        const int fpos = rem ? ic_pos >> 1 : ic_pos, hf = rem ? ic_pos & 1 : 0;
-        if (++ic_pos == (rem ? 2 * NV : NV)) {
-            ++ic_round;
-            ic_pos = 0;
-        }
-        if (withhold != 0 && q == withhold - 1 && blockIdx.x == 0) return;  // test switch: never issued
-        const int s = q % C::NBUF;
-        const unsigned bar = bar0 + 8u * s;
-        mbar_expect_tx(bar, C::BYTES);
-        tma_load_box(smem_addr(ring + (size_t)s * C::SLOT), maps + (size_t)(3 * t.block + in_sel) * 128, t.i0, t.j0,
-                     t.k0 + hf * C::TZ, FIELD_ORDER[fpos], bar);
-    }
-    __device__ __forceinline__ void wait(int q) {
-        if (failed) return;
-        const unsigned bar = bar0 + 8u * (q % C::NBUF), parity = (q / C::NBUF) & 1;
-        if (mbar_try_wait(bar, parity)) return;
-        const unsigned long long t0 = global_ns();
-        for (;;) {
-            if (mbar_try_wait_sleep(bar, parity, TMA_WAIT_HINT_NS)) return;
-            if (global_ns() - t0 > TMA_WAIT_NS) {
-                failed = true;
-                fail_q = q;
+__device__ __forceinline__ void mbar_arrive(unsigned bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
+}
+// Bounded wait for the completion of the phase of parity `parity`; on a timeout
+// the failure is recorded. Returns false then. A waiting warp is suspended
+// within each attempt (mbarrier.try_wait); the clock is read every 64 of them.
+__device__ __forceinline__ bool tma_wait(unsigned bar, unsigned parity, unsigned int* err) {
+    if (mbar_try_wait(bar, parity)) return true;
+    unsigned long long t0 = 0;
+#pragma unroll 1
+    for (unsigned n = 0;; ++n) {
+        if (mbar_try_wait(bar, parity)) return true;
+        if (n % 64 == 0) {
+            const unsigned long long t = global_ns();
+            if (n == 0) t0 = t;
+            if (t - t0 > TMA_WAIT_NS) {
                 if (err) atomicExch(err, 1u);
-                return;
+                return false;
             }
         }
     }
-    // Every thread of the CTA calls der() for every item in order (every BAR-th
-    // call carries the CTA barrier that frees the slots of the last BAR items,
-    // which the next BAR loads overwrite).
-    template <bool HESS, bool EXACT, typename P>
-    __device__ __forceinline__ FieldDer<P> der(int v, const double beta[3], P w) {
-        int q = next;
-        if constexpr (C::REM2) {
-            // a remainder tile's field is two items (one per half): its der()
-            // always starts a barrier group and consumes both
-            if (next % 2 == 0) {
-                __syncthreads();
-                if (threadIdx.x == 0 && !failed) {
-                    issue_next();
-                    issue_next();
-                }
-            }
-            q = next + (rem_round ? half : 0);
-            next += rem_round ? 2 : 1;
-        } else {
-            if (next % C::BAR == 0) {
-                __syncthreads();
-                if (threadIdx.x == 0 && !failed)
-#pragma unroll
-                    for (int j = C::NBUF - C::BAR; j < C::NBUF; ++j) issue(next + j);
-            }
-            ++next;
-        }
-        wait(q);
-        const double* box = ring + (size_t)(q % C::NBUF) * C::SLOT + lin;
-        if constexpr (C::TIN) tin[v * NT] = box[0];
-        const SharedLoad L{box};
-        const long long off[3] = {1, C::BX, C::BX * C::BY};
-        return field_der_l<P, HESS, true, SharedLoad, EXACT>(*B, L, off, beta, w);
+}
+
+// Tile of a compute warpgroup's round r at [r & 1] (index < 0: no more tiles)
+// and its block's descriptor.
+struct __align__(16) TmaTile {
+    Tile t;
+    int index;
+    int pad[2];
+};
+constexpr int TMA_MAX_SLOTS = 4;
+struct TmaShared {
+    unsigned long long full[TMA_MAX_SLOTS], empty[TMA_MAX_SLOTS];
+    TmaTile tile[2];
+    __align__(16) unsigned char block[2][sizeof(DevBlock)];
+};
+static_assert(sizeof(Tile) == 5 * sizeof(int) && sizeof(DevBlock) % 8 == 0 && sizeof(DevBlock) / 8 <= 64,
+              "copied by one warp: a word of the tile and two words of the descriptor per lane");
+__shared__ TmaShared g_tma[4];
+
+// The compute warps' stencil source.
+template <class C, bool UC>
+struct TmaSource {
+    static constexpr bool UNROLL = false;
+    unsigned ring0;  // shared address of the ring
+    const TmaShared& sh;
+    unsigned full0, empty0;
+    const StencilCoef& coef;  // UC: the coefficients of every block of the launch, in the kernel arguments
+    unsigned int* err;
+    int lin = 0;
+    ArmOffsets arm{};
+    int round = 0;
+    int slot = 0;        // ring slot of the next field
+    unsigned phase = 0;  // and the parity of its phase
+    bool failed = false;
+
+    __device__ __forceinline__ const DevBlock& block() const {
+        return *reinterpret_cast<const DevBlock*>(sh.block[round & 1]);
+    }
+    __device__ __forceinline__ void wait() {
+        if (!failed) failed = !tma_wait(full0 + 8u * slot, phase, err);
+    }
+    __device__ __forceinline__ const StencilCoef& coefs() const {
+        if constexpr (UC)
+            return coef;
+        else
+            return block();
+    }
+    template <bool HESS, bool EXACT, bool KOSEP, typename P>
+    __device__ __forceinline__ FieldDer<P> der(int /*v*/, const Advection<P, EXACT>& adv) {
+        wait();
+        const unsigned at = ring0 + slot * (unsigned)(C::SLOT * sizeof(double));
+        const SplitLoad<C::BX, C::BX * C::BY> L{at, at + lin, arm};
+        const FieldDer<P> r = field_der_l<P, HESS, true, EXACT, KOSEP>(coefs(), L, adv);
+        // every lane's loads of the slot come before the warp's arrival
+        __syncwarp();
+        if ((threadIdx.x & 31) == 0) mbar_arrive(empty0 + 8u * slot);
+        if (++slot == C::NBUF) slot = 0, phase ^= 1u;
+        return r;
     }
 };
 
+// The tiles of one compute warpgroup in order: list entries first, first +
+// stride, ..., or with SEL those of them whose flag is `want`. Warp-wide.
+template <bool SEL>
+struct TmaTileFinder {
+    const unsigned char* flags;
+    int want, ntiles, stride;
+    int next;              // next list entry to look at
+    int base = 0;          // SEL: entry of lane 0 of the last 32 looked at
+    unsigned pending = 0;  // and those of them still to be taken
+    __device__ __forceinline__ int find() {
+        if constexpr (SEL) {
+            while (!pending) {
+                if (next >= ntiles) return -1;
+                base = next;
+                const long long ti = base + (long long)(threadIdx.x & 31) * stride;
+                pending = __ballot_sync(0xffffffffu, ti < ntiles && flags[ti] == want);
+                next = (int)min((long long)ntiles, base + 32ll * stride);
+            }
+            const int b = __ffs(pending) - 1;
+            pending &= pending - 1;
+            return base + b * stride;
+        } else {
+            const int t = next;
+            if (t >= ntiles) return -1;
+            next = ntiles - t > stride ? t + stride : ntiles;
+            return t;
+        }
+    }
+};
+
+// One load warp: every lane takes part in the tile search, the copies of tile
+// and descriptor and the waits; lane 0 issues the box loads.
+template <class C, bool SEL>
+__device__ __forceinline__ void tma_load_warp(int g, const DevBlock* __restrict__ blocks, const Tile* __restrict__ tiles,
+                                             int ntiles, const StageArgs& A, unsigned ring0) {
+    TmaShared& sh = g_tma[g];
+    const int lane = threadIdx.x & 31;
+    const unsigned full0 = smem_addr(sh.full), empty0 = smem_addr(sh.empty);
+    constexpr int WORDS = sizeof(DevBlock) / 8;
+    TmaTileFinder<SEL> finder{A.tile_prec, A.want_prec, ntiles, (int)gridDim.x * C::NWG,
+                             (int)(g * gridDim.x + blockIdx.x)};
+    // the tile of the coming round: its list entry, this lane's word of it and this lane's words of the descriptor
+    int ti = finder.find();
+    int tw = ti >= 0 && lane < 5 ? reinterpret_cast<const int*>(tiles + ti)[lane] : 0;
+    unsigned long long d0 = 0, d1 = 0;
+    auto load_desc = [&](int word, unsigned long long& x0, unsigned long long& x1) {
+        const unsigned long long* src =
+            reinterpret_cast<const unsigned long long*>(blocks + __shfl_sync(0xffffffffu, word, 0));
+        x0 = src[lane];
+        if (lane + 32 < WORDS) x1 = src[lane + 32];
+    };
+    if (ti >= 0) load_desc(tw, d0, d1);
+    int slot = 0, q = 0;
+    unsigned ephase = 1;               // parity of the slot's empty phase: the first pass finds the slots empty
+    unsigned issued = 0, parity = 0;   // per slot: a copy was issued into it; the phases its barrier will complete, mod 2
+    bool ok = true;
+    for (int r = 0; ok; ++r) {
+        // (all compute warps have left round r - 2: each arrived on a field of round r - 1)
+        TmaTile& T = sh.tile[r & 1];
+        if (lane < 5) reinterpret_cast<int*>(&T.t)[lane] = tw;
+        if (lane == 5) T.index = ti;
+        unsigned long long* B = reinterpret_cast<unsigned long long*>(sh.block[r & 1]);
+        B[lane] = d0;
+        if (lane + 32 < WORDS) B[lane + 32] = d1;
+        __syncwarp();
+        if (ti < 0) {  // no more tiles: the compute warps see it behind the next slot's barrier
+            if ((ok = tma_wait(empty0 + 8u * slot, ephase, A.errflag)) && lane == 0) {
+                mbar_arrive(full0 + 8u * slot);
+                parity ^= 1u << slot;  // the slot's barrier completes one phase more than its copies
+            }
+            break;
+        }
+        const int blk = __shfl_sync(0xffffffffu, tw, 0), i0 = __shfl_sync(0xffffffffu, tw, 1),
+                  j0 = __shfl_sync(0xffffffffu, tw, 2), k0 = __shfl_sync(0xffffffffu, tw, 3);
+        const bool rem = C::REM && __shfl_sync(0xffffffffu, tw, 4) < 0;
+        const size_t map = (size_t)(3 * blk + A.in_sel) * 128;
+        const unsigned char* m = static_cast<const unsigned char*>(rem ? A.tmaps_rem : A.tmaps) + map;
+        const unsigned char* ma = static_cast<const unsigned char*>(A.tmaps_arm) + map;
+        const int zhi = k0 + (rem ? 2 * C::TZ : C::TZ) + 5;
+        constexpr unsigned ARM = C::Boxes::ARM * sizeof(double);
+        const unsigned arm = (rem ? C::BoxesRem::MAIN : C::Boxes::MAIN) * (unsigned)sizeof(double);
+        const unsigned bytes = (rem ? C::BoxesRem::CELLS : C::Boxes::CELLS) * (unsigned)sizeof(double);
+        ti = finder.find();
+        tw = ti >= 0 && lane < 5 ? reinterpret_cast<const int*>(tiles + ti)[lane] : 0;
+        for (int p = 0; p < NV; ++p) {
+            if (!(ok = tma_wait(empty0 + 8u * slot, ephase, A.errflag))) break;
+            // test switch: item test_withhold - 1 of the first warpgroup is never issued
+            if (lane == 0 && !(A.test_withhold != 0 && q == A.test_withhold - 1 && blockIdx.x == 0 && g == 0)) {
+                const unsigned bar = full0 + 8u * slot, dst = ring0 + slot * (unsigned)(C::SLOT * sizeof(double));
+                const int f = FIELD_ORDER[p];
+                mbar_expect_tx(bar, bytes);
+                // (an interior index is also the cell, incl. ghosts, four lower)
+                tma_load_box(dst, m, i0, j0, k0 + 3, f, bar);
+                tma_load_box(dst + arm, ma, i0 + NG, j0 + NG, k0, f, bar);
+                tma_load_box(dst + arm + ARM, ma, i0 + NG, j0 + NG, zhi, f, bar);
+                issued |= 1u << slot;
+                parity ^= 1u << slot;
+            }
+            __syncwarp();
+            if (++slot == C::NBUF) slot = 0, ephase ^= 1u;
+            ++q;
+            if (p == NV / 2 && ti >= 0) load_desc(tw, d0, d1);
+        }
+    }
+    // no copy into shared memory outlives the CTA: wait for the last one of every slot
+    if (lane == 0)
+        for (int s = 0; s < C::NBUF; ++s)
+            if (issued >> s & 1u) tma_wait(full0 + 8u * s, (parity >> s & 1u) ^ 1u, A.errflag);
+}
+
 }  // namespace
 
-// Persistent CTAs (grid <= SMs x resident CTAs), one 16 x 4 x TZ tile at a
-// time, every field streamed through the TMA ring. Threads of partial tiles
-// (past the block edge) compute on the zero-filled box and store nothing.
-template <int PM, int EPI, class C, bool SEL>
-__global__ void __launch_bounds__(C::NT, C::MINB)
+template <int PM, int EPI, class C, bool SEL, bool UC>
+__global__ void __launch_bounds__(C::NTHR, 1)
     ccz4_stage_tma_kernel(const DevBlock* __restrict__ blocks, const Tile* __restrict__ tiles, int ntiles,
-                          StageArgs A) {
-    using P = typename std::conditional<PM == PM_MIXED, float, double>::type;
-    extern __shared__ unsigned char smem_raw[];
-    unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) &
-                                                           ~uintptr_t(127));
-    double* ring = reinterpret_cast<double*>(base);
-    const unsigned bar0 = smem_addr(base + C::OFF_BAR);
-    const int tid = threadIdx.x;
-    if (tid == 0) {
-        for (int s = 0; s < C::NBUF; ++s) mbar_init(bar0 + 8u * s, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    }
-    // SEL: the CTA's tiles blockIdx.x + m gridDim.x whose flag equals want_prec,
-    // compacted in order into shared memory once (ballot scan over NT candidates
-    // at a time); the host keeps ntiles <= gridDim.x * TMA_SEL_CAP.
-    __shared__ int warp_cnt[C::NT / 32];
-    if constexpr (SEL) {
-        int nsel = 0;
-        const int ncand = ntiles > (int)blockIdx.x ? (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
-        const int lane = tid & 31, warp = tid >> 5;
-        for (int m0 = 0; m0 < ncand; m0 += C::NT) {
-            const int m = m0 + tid;
-            const int ti = blockIdx.x + m * gridDim.x;
-            const bool take = m < ncand && A.tile_prec[ti] == A.want_prec;
-            const unsigned bal = __ballot_sync(0xffffffffu, take);
-            if (lane == 0) warp_cnt[warp] = __popc(bal);
-            __syncthreads();
-            int off = 0, tot = 0;
-#pragma unroll
-            for (int w = 0; w < C::NT / 32; ++w) {
-                off += w < warp ? warp_cnt[w] : 0;
-                tot += warp_cnt[w];
-            }
-            const int pos = nsel + off + __popc(bal & ((1u << lane) - 1u));
-            if (take && pos < TMA_SEL_CAP) g_sel_list[pos] = ti;
-            nsel += tot;
-            __syncthreads();
+                         const __grid_constant__ StageArgs A) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    const int g = threadIdx.x / C::NP;  // warpgroup
+    if (threadIdx.x < C::NWG)
+        for (int s = 0; s < C::NBUF; ++s) {
+            mbar_init(smem_addr(&g_tma[threadIdx.x].full[s]), 1);
+            mbar_init(smem_addr(&g_tma[threadIdx.x].empty[s]), C::NP / 32);  // every compute warp arrives
         }
-        if (tid == 0) g_sel_list[TMA_SEL_CAP] = nsel < TMA_SEL_CAP ? nsel : TMA_SEL_CAP;  // (host keeps it below)
-    }
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     __syncthreads();
-    // push boxes of the current tile, double-buffered by tile round: staged when
-    // the round starts, read in its epilogue (the round's first field barrier
-    // lies between), overwritten two rounds later
-    __shared__ PushBox s_push[2][PUSH_STAGE_MAX];
-    // this thread's point within a tile: 16 x 4 x TZ, or TMA_REM_X x 4 x 2 TZ
-    // for an x-remainder tile (the box rows are the same, so is the stencil code)
-    auto local = [&](const Tile& t, int& px, int& py, int& pz) {
-        if ((C::REM || C::REM2) && t.w < 0) {
-            px = tid % TMA_REM_X;
-            py = (tid / TMA_REM_X) % C::TY;
-            pz = tid / (TMA_REM_X * C::TY);
-        } else {
-            px = tid % C::TX;
-            py = (tid / C::TX) % C::TY;
-            pz = tid / (C::TX * C::TY);
-        }
-    };
-    double* tin = C::TIN ? reinterpret_cast<double*>(base + C::OFF_TIN) + tid : nullptr;
-    void* hs = C::HS ? static_cast<void*>(reinterpret_cast<P*>(base + C::OFF_HS) + tid) : nullptr;
-    TmaSource<C, SEL> S{blocks, tiles, static_cast<const unsigned char*>(A.tmaps),
-                        static_cast<const unsigned char*>(A.tmaps_rem), ntiles, A.in_sel, ring, bar0,
-                        tin, hs, nullptr, 0, 0, false, A.errflag, 0, A.test_withhold};
-    if (tid == 0) {
-        if constexpr (C::REM2)
-            for (int q = 0; q < C::NBUF - C::BAR; ++q) S.issue_next();
-        else
-            for (int q = 0; q < C::NBUF - C::BAR; ++q) S.issue(q);
+    const unsigned rings = smem_addr(smem_raw);
+    constexpr unsigned RING = C::NBUF * C::SLOT * sizeof(double);
+    if (g == C::NWG) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(C::LOAD_REGS));
+        const int w = (threadIdx.x - C::NWG * C::NP) / 32;
+        if (w < C::NWG) tma_load_warp<C, SEL>(w, blocks, tiles, ntiles, A, rings + w * RING);
+        return;
     }
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(C::COMP_REGS));
+    const int pt = threadIdx.x % C::NP;
+    TmaShared& sh = g_tma[g];
+    TmaSource<C, UC> S{rings + g * RING, sh, smem_addr(sh.full), smem_addr(sh.empty), A.coef, A.errflag};
+#pragma unroll 1
     for (int r = 0;; ++r) {
-        const int ti = S.round_tile(r);
-        if (ti >= ntiles) break;
-        const Tile t = tiles[ti];
-        const DevBlock& B = blocks[t.block];
-        S.B = &B;
+        S.wait();  // the round's first field, and with it the tile and its descriptor
+        if (S.failed) break;
+        const Tile t = sh.tile[r & 1].t;
+        const int ti = sh.tile[r & 1].index;
+        if (ti < 0) break;
+        S.round = r;
+        const DevBlock& B = S.block();
+        // this thread's point: 16 x 4 x 2, or TMA_REM_X x 4 x 4 of an x-remainder tile
         int lx, ly, lz;
-        local(t, lx, ly, lz);
-        if constexpr (C::REM2) {
-            // a remainder tile's two halves along z each have their own box
-            S.rem_round = t.w < 0;
-            S.half = S.rem_round ? lz / C::TZ : 0;
-            S.lin = (lx + 4) + C::BX * ((ly + 4) + C::BY * (lz - S.half * C::TZ + 4));
+        if (C::REM && t.w < 0) {
+            lx = pt % TMA_REM_X;
+            ly = (pt / TMA_REM_X) % C::TY;
+            lz = pt / (TMA_REM_X * C::TY);
+            C::BoxesRem::arms(lx, ly, lz, S.arm);
         } else {
-            S.lin = (lx + 4) + C::BX * ((ly + 4) + C::BY * (lz + 4));
+            lx = pt % C::TX;
+            ly = (pt / C::TX) % C::TY;
+            lz = pt / (C::TX * C::TY);
+            C::Boxes::arms(lx, ly, lz, S.arm);
         }
+        S.lin = C::Boxes::point(lx, ly, lz) * (int)sizeof(double);
         const int i = t.i0 + lx, j = t.j0 + ly, k = t.k0 + lz;
         const bool valid = i < B.n[0] && j < B.n[1] && k < B.n[2];
         // pointwise loads of threads outside the block use a valid cell; their results are dropped
         const int ic = min(i, B.n[0] - 1), jc = min(j, B.n[1] - 1), kc = min(k, B.n[2] - 1);
         const long long c = cell_index(B, ic + NG, jc + NG, kc + NG);
-        const double* __restrict__ uin = B.buf[A.in_sel];
-        const PushBox* pushes = nullptr;
-        int npush = 0;
-        if (A.push) {
-            const int2 pr = A.tile_push[ti];
-            npush = pr.y;
-            if (npush <= PUSH_STAGE_MAX) {
-                if (tid < npush) s_push[r & 1][tid] = A.push[pr.x + tid];
-                pushes = s_push[r & 1];
-            } else {
-                pushes = A.push + pr.x;
-            }
-        }
-        if constexpr (C::PF) {
-            // L2 prefetches: this tile's u^n (read by the epilogue; stage 1 takes
-            // it from the ring) and the next tile's pointwise cells
-            if (EPI == EPI_RK && A.n_sel != A.in_sel) {
-                const double* un = B.buf[A.n_sel] + c;
-#pragma unroll
-                for (int v = 0; v < NV; ++v) prefetch_l2(un + (long long)v * B.stride);
-            }
-            const int tn = S.round_tile(r + 1);
-            if (tn < ntiles) {
-                const Tile t2 = tiles[tn];
-                const DevBlock& B2 = blocks[t2.block];
-                int x2, y2, z2;
-                local(t2, x2, y2, z2);
-                const long long c2 = cell_index(B2, min(t2.i0 + x2, B2.n[0] - 1) + NG, min(t2.j0 + y2, B2.n[1] - 1) + NG,
-                                                min(t2.k0 + z2, B2.n[2] - 1) + NG);
-                const double* u2 = B2.buf[A.in_sel] + c2;
-#pragma unroll
-                for (int v = 0; v < NV; ++v) prefetch_l2(u2 + (long long)v * B2.stride);
-            }
-        }
         AlgebraT<PM> L[NV];
-        point_pm<PM>(B, uin, c, A, S, L);
-        if (valid) stage_epilogue<EPI>(B, A, c, L, tin, C::NT, pushes, npush, i, j, k);
-    }
-    // Every issued item was consumed (issue() skips items past this CTA's last
-    // tile), so no copy into the ring is in flight when the CTA exits. If
-    // thread 0 gave up waiting at item f (which already had its full wait), it
-    // had issued items up to f0 + NBUF - 1 (f0 = f rounded down to its barrier
-    // group) and nothing after: each of f + 1 .. f0 + NBUF - 1 that was issued
-    // gets its own bounded wait, whatever the others do, so no copy into this
-    // CTA's shared memory outlives it.
-    if (S.failed && tid == 0) {
-        const int f = S.fail_q;
-        if constexpr (C::REM2) {
-            // the cursor counted every item issued (one the test switch withheld
-            // included: its wait runs out as that of item f did)
-            for (int q = f + 1; q < S.issued; ++q) {
-                S.failed = false;
-                S.wait(q);
-            }
-        } else {
-            for (int q = f + 1; q < f - f % C::BAR + C::NBUF; ++q) {
-                if (S.round_tile(q / NV) >= ntiles) continue;
-                S.failed = false;
-                S.wait(q);
-            }
-        }
+        point_pm<PM>(B, B.buf[A.in_sel], c, A, S, L);
+        const int2 pr = A.push ? A.tile_push[ti] : make_int2(0, 0);
+        if (valid) stage_epilogue<EPI>(B, A, c, L, A.push ? A.push + pr.x : nullptr, pr.y, i, j, k);
+        if (S.failed) break;
     }
 }
 
-// Launchers of one configuration: grids[pm][epi][sel] is the persistent grid
-// (SMs x resident CTAs) measured by tma_configure; 0 = not instantiated.
-template <class C>
-struct TmaConfigOps {
-    template <int PM, int EPI, bool SEL>
+// Launchers of one tile set: C3 the mixed kernels (12 compute warps per SM), C2
+// the FP64 ones (8). grids[pm][epi][sel]: the persistent grid, 0 = not instantiated.
+template <class C3, class C2>
+struct TmaKernelOps {
+    template <int PM>
+    using Cfg = typename std::conditional<PM == PM_MIXED, C3, C2>::type;
+    // the register split needs the launch's full share: setmaxnreg.inc would wait for registers that never free up
+    template <int PM, int EPI, bool SEL, bool UC>
     static cudaError_t configure_one(int nsm, int grids[3][2][2]) {
-        using P = typename std::conditional<PM == PM_MIXED, float, double>::type;
-        auto k = ccz4_stage_tma_kernel<PM, EPI, C, SEL>;
-        constexpr size_t bytes = C::template smem<P>();
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        using C = Cfg<PM>;
+        auto k = ccz4_stage_tma_kernel<PM, EPI, C, SEL, UC>;
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
         if (e != cudaSuccess) return e;
-        int per_sm = 0;
-        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, C::NT, bytes))) return e;
-        grids[PM][EPI][SEL ? 1 : 0] = nsm * (per_sm > 0 ? per_sm : 1);
+        cudaFuncAttributes fa{};
+        if ((e = cudaFuncGetAttributes(&fa, k))) return e;
+        grids[PM][EPI][SEL ? 1 : 0] = fa.numRegs == C::LAUNCH_REGS ? nsm : 0;  // 0: not available
         return cudaSuccess;
     }
-    template <int PM, int EPI, bool SEL>
+    template <int PM, int EPI, bool SEL, bool UC>
     static cudaError_t launch_one(const DevBlock* blocks, const Tile* tiles, int ntiles, const StageArgs& args,
                                   cudaStream_t stream, int grid) {
-        using P = typename std::conditional<PM == PM_MIXED, float, double>::type;
-        ccz4_stage_tma_kernel<PM, EPI, C, SEL>
-            <<<grid, C::NT, C::template smem<P>(), stream>>>(blocks, tiles, ntiles, args);
+        using C = Cfg<PM>;
+        ccz4_stage_tma_kernel<PM, EPI, C, SEL, UC><<<grid, C::NTHR, C::SMEM, stream>>>(blocks, tiles, ntiles, args);
         return cudaGetLastError();
     }
-    // The RK-epilogue kernels every configuration has (FP64; MIXED with and
-    // without per-tile selection; the FP64 pass of the per-tile precision),
-    // plus the store epilogue where STORE is set.
+    template <bool UC>
+    static cudaError_t configure_rk(int nsm, int grids[3][2][2]) {
+        cudaError_t e;
+        if ((e = configure_one<PM_FP64, EPI_RK, false, UC>(nsm, grids))) return e;
+        if ((e = configure_one<PM_MIXED, EPI_RK, false, UC>(nsm, grids))) return e;
+        if ((e = configure_one<PM_MIXED, EPI_RK, true, UC>(nsm, grids))) return e;
+        return configure_one<PM_FP64F, EPI_RK, true, UC>(nsm, grids);
+    }
+    template <bool UC>
+    static cudaError_t launch_rk(int pm, bool sel, const DevBlock* blocks, const Tile* tiles, int ntiles,
+                                 const StageArgs& args, cudaStream_t stream, int grid) {
+        if (pm == PM_FP64 && !sel) return launch_one<PM_FP64, EPI_RK, false, UC>(blocks, tiles, ntiles, args, stream, grid);
+        if (pm == PM_MIXED && !sel) return launch_one<PM_MIXED, EPI_RK, false, UC>(blocks, tiles, ntiles, args, stream, grid);
+        if (pm == PM_MIXED && sel) return launch_one<PM_MIXED, EPI_RK, true, UC>(blocks, tiles, ntiles, args, stream, grid);
+        if (pm == PM_FP64F && sel) return launch_one<PM_FP64F, EPI_RK, true, UC>(blocks, tiles, ntiles, args, stream, grid);
+        return cudaErrorInvalidValue;
+    }
+    // STORE: plus the store epilogue (single-block launches, always uniform).
     template <bool STORE>
     static cudaError_t configure(int nsm, int grids[3][2][2]) {
         cudaError_t e;
-        if ((e = configure_one<PM_FP64, EPI_RK, false>(nsm, grids))) return e;
-        if ((e = configure_one<PM_MIXED, EPI_RK, false>(nsm, grids))) return e;
-        if ((e = configure_one<PM_MIXED, EPI_RK, true>(nsm, grids))) return e;
-        if ((e = configure_one<PM_FP64F, EPI_RK, true>(nsm, grids))) return e;
+        if ((e = configure_rk<false>(nsm, grids))) return e;
+        if ((e = configure_rk<true>(nsm, grids))) return e;
         if constexpr (STORE) {
-            if ((e = configure_one<PM_FP64, EPI_STORE, false>(nsm, grids))) return e;
-            if ((e = configure_one<PM_MIXED, EPI_STORE, false>(nsm, grids))) return e;
+            if ((e = configure_one<PM_FP64, EPI_STORE, false, true>(nsm, grids))) return e;
+            if ((e = configure_one<PM_MIXED, EPI_STORE, false, true>(nsm, grids))) return e;
         }
         return cudaSuccess;
     }
@@ -466,31 +443,16 @@ struct TmaConfigOps {
     static cudaError_t launch(int pm, int epi, bool sel, const DevBlock* blocks, const Tile* tiles, int ntiles,
                               const StageArgs& args, cudaStream_t stream, int grid) {
         if (epi == EPI_RK) {
-            if (pm == PM_FP64 && !sel) return launch_one<PM_FP64, EPI_RK, false>(blocks, tiles, ntiles, args, stream, grid);
-            if (pm == PM_MIXED && !sel) return launch_one<PM_MIXED, EPI_RK, false>(blocks, tiles, ntiles, args, stream, grid);
-            if (pm == PM_MIXED && sel) return launch_one<PM_MIXED, EPI_RK, true>(blocks, tiles, ntiles, args, stream, grid);
-            if (pm == PM_FP64F && sel) return launch_one<PM_FP64F, EPI_RK, true>(blocks, tiles, ntiles, args, stream, grid);
-        } else if constexpr (STORE) {
-            if (pm == PM_FP64 && !sel) return launch_one<PM_FP64, EPI_STORE, false>(blocks, tiles, ntiles, args, stream, grid);
-            if (pm == PM_MIXED && !sel) return launch_one<PM_MIXED, EPI_STORE, false>(blocks, tiles, ntiles, args, stream, grid);
+            if (args.coef_uniform) return launch_rk<true>(pm, sel, blocks, tiles, ntiles, args, stream, grid);
+            return launch_rk<false>(pm, sel, blocks, tiles, ntiles, args, stream, grid);
+        }
+        if constexpr (STORE) {
+            if (!args.coef_uniform || sel) return cudaErrorInvalidValue;
+            if (pm == PM_FP64) return launch_one<PM_FP64, EPI_STORE, false, true>(blocks, tiles, ntiles, args, stream, grid);
+            if (pm == PM_MIXED) return launch_one<PM_MIXED, EPI_STORE, false, true>(blocks, tiles, ntiles, args, stream, grid);
         }
         return cudaErrorInvalidValue;
     }
 };
 
 }  // namespace granite_b200
-
-// One translation unit per configuration k of TMA_CFGS defines its entry points.
-#define GRANITE_TMA_CFG_UNIT(K, STORE)                                                                               \
-    namespace granite_b200 {                                                                                         \
-    using TmaCfg##K =                                                                                                \
-        TmaCfgT<TMA_CFGS[K].tz, TMA_CFGS[K].nbuf, TMA_CFGS[K].tin != 0, TMA_CFGS[K].hs != 0, TMA_CFGS[K].minb,      \
-                TMA_CFGS[K].bar, TMA_CFGS[K].rem, TMA_CFGS[K].pf != 0>;                                              \
-    cudaError_t configure_tma_cfg##K(int nsm, int grids[3][2][2]) {                                                  \
-        return TmaConfigOps<TmaCfg##K>::configure<STORE>(nsm, grids);                                                \
-    }                                                                                                                \
-    cudaError_t launch_tma_cfg##K(int pm, int epi, bool sel, const DevBlock* blocks, const Tile* tiles, int ntiles,  \
-                                  const StageArgs& args, cudaStream_t stream, int grid) {                            \
-        return TmaConfigOps<TmaCfg##K>::launch<STORE>(pm, epi, sel, blocks, tiles, ntiles, args, stream, grid);      \
-    }                                                                                                                \
-    }

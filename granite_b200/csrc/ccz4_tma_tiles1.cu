@@ -1,0 +1,15 @@
+// ccz4_tma_tiles1.cu -- the TMA stage kernel (ccz4_stage_tma.cuh) on tile set 1
+// (ccz4_kernels.h): with x-remainder tiles.
+// Three ring slots per mixed warpgroup leave the per-point body's local memory
+// an L1 of over 70 KB; the FP64 kernels have two warpgroups and take four
+// (456 us with three, 448 with four on 128 x 128 x 64 points).
+#include "ccz4_stage_tma.cuh"
+
+namespace granite_b200 {
+using Ops1 = TmaKernelOps<TmaKernelT<3, 3, true>, TmaKernelT<2, 4, true>>;
+cudaError_t configure_tma_tiles1(int nsm, int grids[3][2][2]) { return Ops1::configure<false>(nsm, grids); }
+cudaError_t launch_tma_tiles1(int pm, int epi, bool sel, const DevBlock* blocks, const Tile* tiles, int ntiles,
+                              const StageArgs& args, cudaStream_t stream, int grid) {
+    return Ops1::launch<false>(pm, epi, sel, blocks, tiles, ntiles, args, stream, grid);
+}
+}  // namespace granite_b200

@@ -394,17 +394,17 @@ GRANITE_API int granite_ccz4_get_kernel_variant(const void* ctx, int* variant);
 
 /* Per-class configurations of GRANITE_VARIANT_TMA (no counterpart in the
  * reference, whose computeRHS runs one OpenMP loop per block, ccz4.cpp:267-270).
- * The TMA stage kernel exists in GRANITE_STAGE_CONFIGS configurations (see
- * granite_ccz4_stage_config_info): tiles of 16 x 4 x tile_z points, ring_slots
- * field boxes in flight, the stage input's centre values kept in shared memory
- * for the RK epilogue (shared_input), the Hessian-field loop's values in shared
- * memory (shared_hessian). Every block belongs to the block-size class whose
- * edge (GRANITE_STAGE_CLASS_EDGES) is nearest on a log scale to the cube root of
- * its interior volume; each (precision, class) has a configuration, the
- * autotuner's B200 winners by default (granite_b200/tuner.py re-tunes and
- * writes a table a caller can apply). A level's blocks of different
- * configurations run as one launch per configuration. Set before commit.
- * All configurations compute identical FP64 results. */
+ * GRANITE_STAGE_CONFIGS configuration ids exist (granite_ccz4_stage_config_info:
+ * the tile depth, ring slots and shared-memory options of the stage kernel each
+ * was a candidate of). The present kernel, whose loads are issued by warps of
+ * their own, is faster than every one of them on every block size and runs for
+ * all ids; an id chooses its tiles: with x-remainder tiles
+ * (granite_ccz4_stage_config_schedule) or without. Every block belongs to the
+ * block-size class whose edge (GRANITE_STAGE_CLASS_EDGES) is nearest on a log
+ * scale to the cube root of its interior volume; each (precision, class) may be
+ * given a configuration; classes without one take the tiles that suit their
+ * level. A level's blocks of different tile sets run as one launch each. Set
+ * before commit. All configurations compute identical FP64 results. */
 #define GRANITE_STAGE_CONFIGS 18
 #define GRANITE_STAGE_CLASSES 6
 #define GRANITE_STAGE_CLASS_EDGES 16, 24, 32, 48, 64, 96
@@ -416,10 +416,8 @@ GRANITE_API int granite_ccz4_get_stage_config(const void* ctx, int precision, in
 GRANITE_API int granite_ccz4_force_stage_config(void* ctx, int cfg);
 GRANITE_API int granite_ccz4_stage_config_info(int cfg, int* tile_z, int* ring_slots, int* shared_input,
                                                int* shared_hessian);
-/* The schedule of a configuration: warp_specialized = 1 when the mixed RK
- * kernels split stencil and algebra warps; ctas_per_sm = the resident CTAs per
- * SM its register allocation is sized for (3: at most 168 registers a thread);
- * items_per_barrier = field boxes consumed per CTA barrier (1 or 2);
+/* The rest of a configuration's description: warp_specialized, ctas_per_sm and
+ * items_per_barrier, of the kernel it was a candidate of (as above);
  * x_remainder_tiles = 1 when a block whose x extent is 8 more than a multiple
  * of 16 covers its last 8 columns with 8 x 4 x 4 tiles instead of 16-wide tiles
  * half outside the block. Null outputs are skipped. */
