@@ -137,9 +137,9 @@ void free_xfer(XferList& x) {
 
 // Inter-level / inter-block transfer lists of one level for one AMR mode.
 struct LevelXfer {
-    XferList prolong;               // into this level from level-1 (ghost slabs, or whole blocks)
-    XferList copy;                  // same-level ghost exchange (GRANITE_AMR_GHOSTS)
-    std::vector<XferList> restrict_;  // into this level from level+1; one list per launch
+    XferList prolong;               // into this level from level-1 (whole blocks, REFERENCE)
+    GhostSrc* d_restrict = nullptr; // into this level from level+1: each restricted cell once
+    long long nrestrict = 0;
     unsigned char* d_facemask = nullptr;  // faces left to the zero-gradient fill (REFERENCE)
     GhostSrc* d_src = nullptr;            // one source per ghost cell of the level (GHOSTS)
     long long nsrc = 0;
@@ -1119,8 +1119,7 @@ static void release_lists(Ctx* c) {
     for (int m = 0; m < 2; ++m) {
         for (auto& X : c->xfer[m]) {
             free_xfer(X.prolong);
-            free_xfer(X.copy);
-            for (auto& r : X.restrict_) free_xfer(r);
+            cudaFree(X.d_restrict);
             cudaFree(X.d_facemask);
             cudaFree(X.d_src);
             cudaFree(X.d_src_stage);
@@ -1345,7 +1344,7 @@ int granite_ccz4_regrid_add(void* h, const granite_block_desc* b, int n) {
         for (int d = 0; d < 3; ++d) x.n[d] = b[i].ncells[d] + 2 * NG;
         XferList xl;
         e = upload_xfer(std::vector<XferBox>{x}, xl, c->stream);
-        if (e == cudaSuccess) e = launch_xfer(XFER_PROLONG, d_hb, xl.d_boxes, xl.d_chunks, xl.nchunks, 0, 0, c->stream);
+        if (e == cudaSuccess) e = launch_prolong(d_hb, xl.d_boxes, xl.d_chunks, xl.nchunks, 0, 0, c->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
         free_xfer(xl);
     }
@@ -1688,6 +1687,36 @@ int level_grid(Ctx* c, std::vector<std::array<int, 3>>& G) {
     return GRANITE_OK;
 }
 
+// The restriction boxes into a level (x.dst coarse, x.src fine, children of the
+// box's first cell at x.s0) as one list with each coarse cell once: where boxes
+// overlap the last one decides, as when they run one after the other (a box
+// reads only cells of the finer level).
+int upload_restriction(Ctx* c, const std::vector<XferBox>& boxes, LevelXfer& X) {
+    std::map<int, std::vector<GhostSrc>> cells;  // per coarse block
+    for (const XferBox& x : boxes) {
+        const auto& d = c->descs[x.dst];
+        const auto& f = c->descs[x.src];
+        const int T0 = d.ncells[0] + 2 * NG, T1 = d.ncells[1] + 2 * NG, T2 = d.ncells[2] + 2 * NG;
+        const int S0 = f.ncells[0] + 2 * NG, S1 = f.ncells[1] + 2 * NG;
+        auto& m = cells[x.dst];
+        if (m.empty()) m.assign((size_t)T0 * T1 * T2, GhostSrc{-1, 0, 0, 0});
+        for (int k = 0; k < x.n[2]; ++k)
+            for (int j = 0; j < x.n[1]; ++j)
+                for (int i = 0; i < x.n[0]; ++i) {
+                    const int cell = x.d0[0] + i + T0 * (x.d0[1] + j + T1 * (x.d0[2] + k));
+                    m[cell] = GhostSrc{x.dst, cell, x.src,
+                                       x.s0[0] + 2 * i + S0 * (x.s0[1] + 2 * j + S1 * (x.s0[2] + 2 * k))};
+                }
+    }
+    std::vector<GhostSrc> items;
+    for (const auto& kv : cells)
+        for (const GhostSrc& g : kv.second)
+            if (g.dst_block >= 0) items.push_back(g);
+    CK(upload_vec(items, &X.d_restrict, c->stream), "upload restriction list");
+    X.nrestrict = (long long)items.size();
+    return GRANITE_OK;
+}
+
 // Transfer lists for GRANITE_AMR_GHOSTS: ghost slabs of every fine block filled
 // from the coarse blocks covering them, then overwritten by same-level
 // neighbours where one covers the cell; coarse cells whose 2x2x2 children lie
@@ -1726,7 +1755,6 @@ int build_ghosts_mode(Ctx* c) {
                 x.src = b;
                 copies.push_back(x);
             }
-        CK(upload_xfer(copies, X[L].copy, c->stream), "upload copy boxes");
         // prolongation into the six ghost slabs of each fine block
         std::vector<XferBox> pro;
         for (int f : (L > 0 ? blocks : std::vector<int>())) {
@@ -1765,7 +1793,6 @@ int build_ghosts_mode(Ctx* c) {
                 }
             }
         }
-        CK(upload_xfer(pro, X[L].prolong, c->stream), "upload prolongation boxes");
         // one source per ghost cell: same-level neighbour over coarse block over own fill
         {
             std::vector<GhostSrc> items, sitems;
@@ -1907,26 +1934,13 @@ int build_ghosts_mode(Ctx* c) {
                 if (!X[L].d_push) X[L].push_ok = false;  // nothing to push on this level
             }
         }
-        // restriction into level L-1 from level L: one launch for the level, or,
-        // where fine interiors overlap (a regrid adds blocks beside the old ones),
-        // one launch per fine block in list order so that the last one holding a
-        // coarse cell's children decides it, as in the reference (amr.cpp:339-341)
+        // restriction into level L-1 from level L, fine block by fine block in list
+        // order: where fine interiors overlap (a regrid adds blocks beside the old
+        // ones) the last one holding a coarse cell's children decides it, as in the
+        // reference (amr.cpp:339-341)
         if (L == 0) continue;
-        bool overlap = false;
-        for (size_t p = 0; p < blocks.size() && !overlap; ++p)
-            for (size_t q = p + 1; q < blocks.size() && !overlap; ++q) {
-                bool all = true;
-                for (int d = 0; d < 3 && all; ++d)
-                    all = !meet({G[blocks[p]][d], G[blocks[p]][d] + c->descs[blocks[p]].ncells[d]},
-                                {G[blocks[q]][d], G[blocks[q]][d] + c->descs[blocks[q]].ncells[d]})
-                               .empty();
-                overlap = all;
-            }
-        std::vector<std::vector<XferBox>> waves(overlap ? blocks.size() : 1);
-        for (int cb : c->levels[L - 1].blocks)
-            for (size_t fi = 0; fi < blocks.size(); ++fi) {
-                const int f = blocks[fi];
-                std::vector<XferBox>& res = waves[overlap ? fi : 0];
+        for (int f : blocks)
+            for (int cb : c->levels[L - 1].blocks) {
                 XferBox x{};
                 bool ok = true;
                 for (int d = 0; d < 3; ++d) {
@@ -1945,13 +1959,9 @@ int build_ghosts_mode(Ctx* c) {
                 if (!ok) continue;
                 x.dst = cb;
                 x.src = f;
-                res.push_back(x);
+                restricted[L - 1].push_back(x);
             }
-        for (const auto& res : waves) {
-            X[L - 1].restrict_.emplace_back();
-            CK(upload_xfer(res, X[L - 1].restrict_.back(), c->stream), "upload restriction boxes");
-            for (const XferBox& x : res) restricted[L - 1].push_back(x);
-        }
+        if ((r = upload_restriction(c, restricted[L - 1], X[L - 1]))) return r;
     }
     // The fill before a level step when the same-level copies are current (the
     // fill after the level's previous step, or its pushing stages, made them
@@ -2027,10 +2037,11 @@ int build_reference_mode(Ctx* c) {
                 mask[f] = m;
             }
             CK(upload_xfer(pro, X[L].prolong, c->stream), "upload prolongation boxes");
-            // restriction into level L-1, one launch per fine block in order
+            // restriction into level L-1, fine block by fine block in order (a box reaches
+            // into its block's upper ghost layer, so neighbours' boxes overlap)
+            std::vector<XferBox> res;
             for (int f : blocks) {
                 const auto& fd = c->descs[f];
-                std::vector<XferBox> res;
                 for (int cb : c->levels[L - 1].blocks) {
                     const auto& cd = c->descs[cb];
                     XferBox x{};
@@ -2065,9 +2076,9 @@ int build_reference_mode(Ctx* c) {
                     x.src = f;
                     res.push_back(x);
                 }
-                X[L - 1].restrict_.emplace_back();
-                CK(upload_xfer(res, X[L - 1].restrict_.back(), c->stream), "upload restriction boxes");
             }
+            int r = upload_restriction(c, res, X[L - 1]);
+            if (r) return r;
         }
         CK(upload_vec(mask, &X[L].d_facemask, c->stream), "upload face masks");
     }
@@ -2075,10 +2086,10 @@ int build_reference_mode(Ctx* c) {
     return GRANITE_OK;
 }
 
-cudaError_t xfer(Ctx* c, int kind, const XferList& x, int dst_sel, int src_sel) {
+cudaError_t prolong(Ctx* c, const XferList& x, int dst_sel, int src_sel) {
     if (x.nchunks == 0) return cudaSuccess;
     return timed(c, GRANITE_KERNEL_TRANSFER, [&] {
-        return launch_xfer(kind, c->d_blocks, x.d_boxes, x.d_chunks, x.nchunks, dst_sel, src_sel, c->stream);
+        return launch_prolong(c->d_blocks, x.d_boxes, x.d_chunks, x.nchunks, dst_sel, src_sel, c->stream);
     });
 }
 
@@ -2087,15 +2098,17 @@ cudaError_t xfer(Ctx* c, int kind, const XferList& x, int dst_sel, int src_sel) 
 // pushed: the fill after a stage that pushed the same-level copies (no copies);
 // prefill_fresh: the fill before a step while the pushed copies are current
 // (only the copies of cells restrictions write).
-cudaError_t fill_level(Ctx* c, int L, int slot, bool level_fill, int mode, long long* n, bool pushed = false,
-                       bool prefill_fresh = false) {
+// prolong: GRANITE_AMR_GHOSTS, the slots from `slot` on that the prolongated
+// cells are written in (0: they hold their values).
+cudaError_t fill_level(Ctx* c, int L, int slot, bool level_fill, int mode, long long* n, int prolong_slots,
+                       bool pushed = false, bool prefill_fresh = false) {
     LevelLists& ll = c->levels[L];
     const LevelXfer& X = c->xfer[mode][L];
     cudaError_t e;
     if (mode == GRANITE_AMR_REFERENCE) {
         if (level_fill) {
             if (L > 0) {  // fillGhostZones: prolongate into all cells, then the uncovered faces
-                if ((e = xfer(c, XFER_PROLONG, X.prolong, slot, 0))) return e;
+                if ((e = prolong(c, X.prolong, slot, 0))) return e;
                 ++*n;
             }
             const int gm = L > 0 ? GHOST_ZERO_GRADIENT_MASKED : GHOST_ZERO_GRADIENT;
@@ -2121,14 +2134,14 @@ cudaError_t fill_level(Ctx* c, int L, int slot, bool level_fill, int mode, long 
         if (nsrc == 0) return cudaSuccess;
         ++*n;
         return timed(c, GRANITE_KERNEL_GHOST, [&] {
-            return launch_ghost_sources(c->d_blocks, src, nsrc, slot, local, c->stream);
+            return launch_ghost_sources(c->d_blocks, src, nsrc, slot, local, prolong_slots, c->stream);
         });
     }
     for (const auto& r : ranges) {
         if (r.second == 0) continue;
         ++*n;
         if ((e = timed(c, GRANITE_KERNEL_GHOST, [&] {
-                 return launch_ghost_sources(c->d_blocks, src + r.first, r.second, slot, local, c->stream);
+                 return launch_ghost_sources(c->d_blocks, src + r.first, r.second, slot, local, prolong_slots, c->stream);
              })))
             return e;
     }
@@ -2179,17 +2192,25 @@ struct RegridHook {
 // runs at the reference's regrid points.
 // skip_prefill: the level's state and every cell its fill reads are what the
 // fill at the end of its previous step saw (the second substep of the finest
-// level in GRANITE_AMR_GHOSTS: nothing restricts into it, its parent does not
-// change between the two substeps), so the fill before this step would write
-// the values already there.
+// level: nothing restricts into it, its parent does not change between the two
+// substeps), so the fill before this step would write the values already there
+// (in GRANITE_AMR_REFERENCE also the prolongation of the whole level).
+// substep: which of the two substeps within the parent's step this is. The
+// ghost cells a level takes from its parent (GRANITE_AMR_GHOSTS) do not change
+// within the pair: they are prolongated from the parent's slot 0, which only
+// the restriction after the pair writes, and no stage writes ghost cells. So the
+// first substep's fill writes them into all three slots and the other fills of
+// the pair leave them (7 of 8 fills; a third of the cells a fill of the 3-level
+// test hierarchy wrote). With a regrid hook the arena may move in between:
+// every fill prolongates.
 cudaError_t subcycle(Ctx* c, int L, double dt, int precision, int mode, long long* n, RegridHook* hook = nullptr,
-                     bool skip_prefill = false) {
+                     int substep = 0, bool skip_prefill = false) {
     cudaError_t e;
     if (hook && (hook->status = ensure_xfer(c, mode))) return cudaErrorInvalidValue;
     const LevelXfer& X = c->xfer[mode][L];
     if (skip_prefill) {
     } else if (mode == GRANITE_AMR_REFERENCE && L > 0) {  // amr.cpp:313-318 (the fill below repeats it exactly)
-        if ((e = xfer(c, XFER_PROLONG, X.prolong, 0, 0))) return e;
+        if ((e = prolong(c, X.prolong, 0, 0))) return e;
         ++*n;
         if ((e = level_ghost(c, c->levels[L], GHOST_ZERO_GRADIENT_MASKED, 0, X.d_facemask, n))) return e;
     } else {
@@ -2199,29 +2220,33 @@ cudaError_t subcycle(Ctx* c, int L, double dt, int precision, int mode, long lon
         // the level's state changed only by restrictions into it
         const bool fresh = mode == GRANITE_AMR_GHOSTS &&
                            (c->copies_valid || (L < (int)c->step_pushed.size() && c->step_pushed[L]));
-        if ((e = fill_level(c, L, 0, true, mode, n, false, fresh))) return e;
+        if ((e = fill_level(c, L, 0, true, mode, n, hook ? 1 : (substep == 0 ? 3 : 0), false, fresh))) return e;
     }
+    const int pro = hook ? 1 : 0;
     // TimeIntegrator::sspRK3Step, main.cpp:673-689 (in GRANITE_AMR_GHOSTS the
     // stages write the same-level ghost copies themselves; the fills add the rest)
     const bool push = pushes(c, L, mode);
     if ((e = stage(c, L, precision, 0, 1, 1.0, 0.0, 1.0 * dt, 0, n, push))) return e;
-    if ((e = fill_level(c, L, 1, false, mode, n, push))) return e;
+    if ((e = fill_level(c, L, 1, false, mode, n, pro, push))) return e;
     if ((e = stage(c, L, precision, 1, 2, 0.75, 0.25, 0.25 * dt, 0, n, push))) return e;
-    if ((e = fill_level(c, L, 2, false, mode, n, push))) return e;
+    if ((e = fill_level(c, L, 2, false, mode, n, pro, push))) return e;
     if ((e = stage(c, L, precision, 2, 0, 1.0 / 3.0, 2.0 / 3.0, (2.0 / 3.0) * dt, 1, n, push))) return e;
-    if ((e = fill_level(c, L, 0, true, mode, n, push))) return e;  // amr.cpp:329
+    if ((e = fill_level(c, L, 0, true, mode, n, pro, push))) return e;  // amr.cpp:329
     if (mode == GRANITE_AMR_GHOSTS && L < (int)c->step_pushed.size()) c->step_pushed[L] = 1;
     if (hook) c->level_time[L] += dt;                         // amr.cpp:326
     if (L + 1 < (int)c->levels.size()) {
         for (int r = 0; r < 2; ++r) {  // amr.cpp:334-336, :393-397
             // (with a regrid hook the level list may change between the substeps: always fill)
-            const bool skip = r == 1 && !hook && mode == GRANITE_AMR_GHOSTS && L + 2 == (int)c->levels.size();
-            if ((e = subcycle(c, L + 1, dt / 2.0, precision, mode, n, hook, skip))) return e;
+            const bool skip = r == 1 && !hook && L + 2 == (int)c->levels.size();
+            if ((e = subcycle(c, L + 1, dt / 2.0, precision, mode, n, hook, r, skip))) return e;
         }
         if (hook && (hook->status = ensure_xfer(c, mode))) return cudaErrorInvalidValue;  // a regrid rebuilt them
-        for (const XferList& rl : c->xfer[mode][L].restrict_) {                            // amr.cpp:339-341
-            if ((e = xfer(c, XFER_RESTRICT, rl, 0, 0))) return e;
+        const LevelXfer& XL = c->xfer[mode][L];
+        if (XL.nrestrict > 0) {  // amr.cpp:339-341
             ++*n;
+            if ((e = timed(c, GRANITE_KERNEL_TRANSFER,
+                           [&] { return launch_restrict(c->d_blocks, XL.d_restrict, XL.nrestrict, c->stream); })))
+                return e;
         }
     }
     if (hook && hook->interval > 0) {

@@ -72,6 +72,35 @@ __device__ FalloffChain falloff_chain(const DevBlock& B, int i, int j, int k) {
     return ch;
 }
 
+// All fields of a cell, in two batches.
+__device__ __forceinline__ void copy_cell(double* dst, long long dstr, const double* src, long long sstr) {
+#pragma unroll
+    for (int h = 0; h < NV; h += NV / 2) {
+        double v_[NV / 2];
+#pragma unroll
+        for (int v = 0; v < NV / 2; ++v) v_[v] = __ldg(src + (h + v) * sstr);
+#pragma unroll
+        for (int v = 0; v < NV / 2; ++v) dst[(h + v) * dstr] = v_[v];
+    }
+}
+__device__ __forceinline__ void falloff_cell(double* base, long long stride, long long dst, const FalloffChain& ch) {
+#pragma unroll
+    for (int h = 0; h < NV; h += NV / 2) {
+        double v_[NV / 2];
+#pragma unroll
+        for (int v = 0; v < NV / 2; ++v) v_[v] = __ldg(base + (h + v) * stride + ch.src);
+#pragma unroll
+        for (int v = 0; v < NV / 2; ++v) {
+            const double fi = f_inf(h + v);
+            double val = v_[v];
+#pragma unroll
+            for (int p = 0; p < 3; ++p)  // unrolled with a guard: the radii stay in registers
+                if (p < ch.npass) val = falloff(fi, val, ch.ri[p], ch.rg[p]);
+            base[(h + v) * stride + dst] = val;
+        }
+    }
+}
+
 // r-th ghost cell of a block: z slabs first, then y slabs, then x slabs.
 __device__ __forceinline__ bool ghost_coords(const DevBlock& B, long long r, int& i, int& j, int& k) {
     const int T0 = B.tx, T1 = B.ty;
@@ -117,8 +146,9 @@ __device__ __forceinline__ int masked_clamp(int a, int n, unsigned mask, int axi
     return a;
 }
 
-// items[x].cell holds the first ghost rank of a chunk of blockDim.x ranks.
-__global__ void ghost_fill_kernel(int mode, const DevBlock* __restrict__ blocks, const GhostItem* __restrict__ items,
+// items[x].cell holds the first ghost rank of a chunk of blockDim.x ranks. The
+// cells a launch reads (interior cells) are never written by it.
+__global__ void __launch_bounds__(256, 4) ghost_fill_kernel(int mode, const DevBlock* __restrict__ blocks, const GhostItem* __restrict__ items,
                                   int sel, const unsigned char* __restrict__ facemask) {
     const GhostItem it = items[blockIdx.x];
     const DevBlock& B = blocks[it.block];
@@ -127,15 +157,7 @@ __global__ void ghost_fill_kernel(int mode, const DevBlock* __restrict__ blocks,
     double* base = B.buf[sel];
     const long long c = cell_index(B, i, j, k);
     if (mode == GHOST_SOMMERFELD) {
-        const FalloffChain ch = falloff_chain(B, i, j, k);
-        for (int v = 0; v < NV; ++v) {
-            const double fi = f_inf(v);
-            double val = base[(long long)v * B.stride + ch.src];
-#pragma unroll
-            for (int p = 0; p < 3; ++p)  // unrolled with a guard: the radii stay in registers
-                if (p < ch.npass) val = falloff(fi, val, ch.ri[p], ch.rg[p]);
-            base[(long long)v * B.stride + c] = val;
-        }
+        falloff_cell(base, B.stride, c, falloff_chain(B, i, j, k));
         return;
     }
     int si, sj, sk;
@@ -154,15 +176,17 @@ __global__ void ghost_fill_kernel(int mode, const DevBlock* __restrict__ blocks,
         sj = j < NG ? j + B.n[1] : (j >= NG + B.n[1] ? j - B.n[1] : j);
         sk = k < NG ? k + B.n[2] : (k >= NG + B.n[2] ? k - B.n[2] : k);
     }
-    const long long s = cell_index(B, si, sj, sk);
-    for (int v = 0; v < NV; ++v) base[(long long)v * B.stride + c] = base[(long long)v * B.stride + s];
+    copy_cell(base + c, B.stride, base + cell_index(B, si, sj, sk), B.stride);
 }
 
 // Trilinear prolongation of coarse block C into fine cell (i,j,k) of F,
 // amr.cpp:496-561: nearest coarse centre by rounding, one-sided neighbour by
 // the sign of the fractional offset, indices clamped to the coarse block.
-__device__ void prolong_cell(const DevBlock& F, const DevBlock& C, int i, int j, int k, double* __restrict__ fb,
-                             const double* __restrict__ cb) {
+// Fields [v0, v0 + nv); writes nslot slots of F from slot sel on (the same value
+// in each). U fields' loads (8 each) are in flight at a time.
+template <int U>
+__device__ __forceinline__ void prolong_cell(const DevBlock& F, const DevBlock& C, int i, int j, int k, int sel, int nslot,
+                                             const double* __restrict__ cb, int v0, int nv) {
     const int fi[3] = {i, j, k};
     const int ct[3] = {C.tx, C.ty, C.tz};
     int c0[3], c1[3];
@@ -194,8 +218,8 @@ __device__ void prolong_cell(const DevBlock& F, const DevBlock& C, int i, int j,
     const int o110 = (int)cell_index(C, c1[0], c1[1], c0[2]), o101 = (int)cell_index(C, c1[0], c0[1], c1[2]);
     const int o011 = (int)cell_index(C, c0[0], c1[1], c1[2]), o111 = (int)cell_index(C, c1[0], c1[1], c1[2]);
     const long long fc = cell_index(F, i, j, k);
-#pragma unroll 2
-    for (int v = 0; v < NV; ++v) {
+#pragma unroll U
+    for (int v = v0; v < v0 + nv; ++v) {
         const double* q = cb + (long long)v * C.stride;
         double val = __dmul_rn(w000, __ldg(q + o000));
         val = __dadd_rn(val, __dmul_rn(w100, __ldg(q + o100)));
@@ -205,42 +229,51 @@ __device__ void prolong_cell(const DevBlock& F, const DevBlock& C, int i, int j,
         val = __dadd_rn(val, __dmul_rn(w101, __ldg(q + o101)));
         val = __dadd_rn(val, __dmul_rn(w011, __ldg(q + o011)));
         val = __dadd_rn(val, __dmul_rn(w111, __ldg(q + o111)));
-        fb[(long long)v * F.stride + fc] = val;
+        for (int s = 0; s < nslot; ++s) F.buf[sel + s][(long long)v * F.stride + fc] = val;
     }
 }
 
-__global__ void xfer_kernel(int kind, const DevBlock* __restrict__ blocks, const XferBox* __restrict__ boxes,
-                            const BoxChunk* __restrict__ chunks, int dst_sel, int src_sel) {
+// Prolongation of whole boxes: a thread per cell and half of the fields (blockIdx.y).
+__global__ void __launch_bounds__(XFER_CHUNK, 2)
+    prolong_kernel(const DevBlock* __restrict__ blocks, const XferBox* __restrict__ boxes,
+                   const BoxChunk* __restrict__ chunks, int dst_sel, int src_sel) {
     const BoxChunk ch = chunks[blockIdx.x];
     const XferBox bx = boxes[ch.box];
     const int r = ch.start + threadIdx.x;
     if (r >= bx.n[0] * bx.n[1] * bx.n[2]) return;
     const int a = r % bx.n[0], b = (r / bx.n[0]) % bx.n[1], c = r / (bx.n[0] * bx.n[1]);
-    const DevBlock& D = blocks[bx.dst];
     const DevBlock& S = blocks[bx.src];
-    const int i = bx.d0[0] + a, j = bx.d0[1] + b, k = bx.d0[2] + c;
-    double* db = D.buf[dst_sel];
-    const double* sb = S.buf[src_sel];
-    if (kind == XFER_PROLONG) {
-        prolong_cell(D, S, i, j, k, db, sb);
-        return;
-    }
-    const long long dc = cell_index(D, i, j, k);
-    if (kind == XFER_COPY) {
-        const long long sc = cell_index(S, bx.s0[0] + a, bx.s0[1] + b, bx.s0[2] + c);
-        for (int v = 0; v < NV; ++v) db[(long long)v * D.stride + dc] = __ldg(sb + (long long)v * S.stride + sc);
-        return;
-    }
-    // restriction: mean of the 2x2x2 fine cells, summed rk, rj, ri (amr.cpp:601-609)
-    const long long f0 = cell_index(S, bx.s0[0] + 2 * a, bx.s0[1] + 2 * b, bx.s0[2] + 2 * c);
+    prolong_cell<4>(blocks[bx.dst], S, bx.d0[0] + a, bx.d0[1] + b, bx.d0[2] + c, dst_sel, 1, S.buf[src_sel],
+                    blockIdx.y * (NV / 2), NV / 2);
+}
+
+// Restriction: mean of the 2x2x2 fine cells, summed rk, rj, ri (amr.cpp:601-609).
+// One thread per listed coarse cell and RESTRICT_FIELDS fields (blockIdx.y), so a
+// level of 64^3 cells is 1408 CTAs. A list holds each coarse cell once.
+constexpr int RESTRICT_FIELDS = 2;
+__global__ void __launch_bounds__(256) restrict_kernel(const DevBlock* __restrict__ blocks,
+                                                       const GhostSrc* __restrict__ items, long long n) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const GhostSrc it = items[t];
+    const DevBlock& D = blocks[it.dst_block];
+    const DevBlock& S = blocks[it.src_block];
     const long long sx = 1, sy = S.tx, sz = (long long)S.tx * S.ty;
-    for (int v = 0; v < NV; ++v) {
-        const double* q = sb + (long long)v * S.stride + f0;
+    const int v0 = blockIdx.y * RESTRICT_FIELDS;
+    double* d = D.buf[0] + v0 * D.stride + it.dst_cell;
+    const double* q = S.buf[0] + v0 * S.stride + it.src_cell;
+    double f[RESTRICT_FIELDS][8];
+#pragma unroll
+    for (int v = 0; v < RESTRICT_FIELDS; ++v)
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+            f[v][r] = __ldg(q + v * S.stride + (r & 1) * sx + (r >> 1 & 1) * sy + (r >> 2) * sz);
+#pragma unroll
+    for (int v = 0; v < RESTRICT_FIELDS; ++v) {
         double s = 0.0;
-        for (int rk = 0; rk < 2; ++rk)
-            for (int rj = 0; rj < 2; ++rj)
-                for (int ri = 0; ri < 2; ++ri) s = __dadd_rn(s, __ldg(q + ri * sx + rj * sy + rk * sz));
-        db[(long long)v * D.stride + dc] = __ddiv_rn(s, 8.0);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) s = __dadd_rn(s, f[v][r]);
+        d[v * D.stride] = __dmul_rn(s, 0.125);  // the rounding of s / 8.0
     }
 }
 
@@ -251,66 +284,50 @@ __global__ void xfer_kernel(int kind, const DevBlock* __restrict__ blocks, const
 // two halves and the prolongation keeps 32-bit offsets, so the paths fit without
 // the 127 registers (16 warps per SM) of a one-pass version; about 5 % faster on
 // the hierarchy's fills.
+// prolong: the slots from sel on that prolongated cells are written in (0: they
+// are left out).
 __global__ void __launch_bounds__(256, 4) ghost_sources_kernel(const DevBlock* __restrict__ blocks, const GhostSrc* __restrict__ items,
-                                     long long n, int sel, int local_mode) {
+                                     long long n, int sel, int local_mode, int prolong) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     const GhostSrc it = items[t];
+    const bool coarse = it.src_block >= 0 && it.src_cell < 0;
+    if (coarse && prolong == 0) return;
     const DevBlock& D = blocks[it.dst_block];
     double* db = D.buf[sel];
-    const long long dst = it.dst_cell, dstr = D.stride;
-    const int i = it.dst_cell % D.tx, j = (it.dst_cell / D.tx) % D.ty, k = it.dst_cell / (D.tx * D.ty);
-    if (it.src_block >= 0 && it.src_cell < 0) {  // coarse level
-        const DevBlock& C = blocks[it.src_block];
-        prolong_cell(D, C, i, j, k, db, C.buf[0]);
-        return;
-    }
-    const double* src;
-    long long sstr;
-    if (it.src_block >= 0) {  // same-level neighbour
+    if (it.src_block >= 0 && !coarse) {  // same-level neighbour
         const DevBlock& S = blocks[it.src_block];
-        src = S.buf[sel] + it.src_cell;
-        sstr = S.stride;
-    } else if (local_mode == GHOST_SOMMERFELD) {
-        const FalloffChain ch = falloff_chain(D, i, j, k);
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            double v_[NV / 2];
-#pragma unroll
-            for (int v = 0; v < NV / 2; ++v) v_[v] = __ldg(db + (h * (NV / 2) + v) * dstr + ch.src);
-#pragma unroll
-            for (int v = 0; v < NV / 2; ++v) {
-                const double fi = f_inf(h * (NV / 2) + v);
-                double val = v_[v];
-    #pragma unroll
-            for (int p = 0; p < 3; ++p)  // unrolled with a guard: the radii stay in registers
-                if (p < ch.npass) val = falloff(fi, val, ch.ri[p], ch.rg[p]);
-                db[(h * (NV / 2) + v) * dstr + dst] = val;
-            }
-        }
+        copy_cell(db + it.dst_cell, D.stride, S.buf[sel] + it.src_cell, S.stride);
         return;
-    } else {  // zero gradient
-        src = db + cell_index(D, clampi(i, NG, NG + D.n[0] - 1), clampi(j, NG, NG + D.n[1] - 1),
-                              clampi(k, NG, NG + D.n[2] - 1));
-        sstr = dstr;
     }
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        double v_[NV / 2];
-#pragma unroll
-        for (int v = 0; v < NV / 2; ++v) v_[v] = __ldg(src + (h * (NV / 2) + v) * sstr);
-#pragma unroll
-        for (int v = 0; v < NV / 2; ++v) db[(h * (NV / 2) + v) * dstr + dst] = v_[v];
+    const int i = it.dst_cell % D.tx, j = (it.dst_cell / D.tx) % D.ty, k = it.dst_cell / (D.tx * D.ty);
+    if (coarse) {
+        const DevBlock& C = blocks[it.src_block];
+        prolong_cell<2>(D, C, i, j, k, sel, prolong, C.buf[0], 0, NV);
+    } else if (local_mode == GHOST_SOMMERFELD) {
+        falloff_cell(db, D.stride, it.dst_cell, falloff_chain(D, i, j, k));
+    } else {  // zero gradient
+        copy_cell(db + it.dst_cell, D.stride,
+                  db + cell_index(D, clampi(i, NG, NG + D.n[0] - 1), clampi(j, NG, NG + D.n[1] - 1),
+                                  clampi(k, NG, NG + D.n[2] - 1)),
+                  D.stride);
     }
 }
 
 }  // namespace
 
 cudaError_t launch_ghost_sources(const DevBlock* blocks, const GhostSrc* items, long long nitems, int sel,
-                                 int local_mode, cudaStream_t stream) {
+                                 int local_mode, int prolong, cudaStream_t stream) {
     if (nitems <= 0) return cudaSuccess;
-    ghost_sources_kernel<<<(unsigned)((nitems + 255) / 256), 256, 0, stream>>>(blocks, items, nitems, sel,
-                                                                            local_mode);
+    ghost_sources_kernel<<<(unsigned)((nitems + 255) / 256), 256, 0, stream>>>(blocks, items, nitems, sel, local_mode,
+                                                                            prolong);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_restrict(const DevBlock* blocks, const GhostSrc* items, long long nitems, cudaStream_t stream) {
+    if (nitems <= 0) return cudaSuccess;
+    static_assert(NV % RESTRICT_FIELDS == 0, "field groups");
+    restrict_kernel<<<dim3((unsigned)((nitems + 255) / 256), NV / RESTRICT_FIELDS), 256, 0, stream>>>(blocks, items, nitems);
     return cudaGetLastError();
 }
 
@@ -323,10 +340,10 @@ cudaError_t launch_ghost_fill(int mode, const DevBlock* blocks, const GhostItem*
     return cudaGetLastError();
 }
 
-cudaError_t launch_xfer(int kind, const DevBlock* blocks, const XferBox* boxes, const BoxChunk* chunks, int nchunks,
-                        int dst_sel, int src_sel, cudaStream_t stream) {
+cudaError_t launch_prolong(const DevBlock* blocks, const XferBox* boxes, const BoxChunk* chunks, int nchunks, int dst_sel,
+                           int src_sel, cudaStream_t stream) {
     if (nchunks <= 0) return cudaSuccess;
-    xfer_kernel<<<nchunks, XFER_CHUNK, 0, stream>>>(kind, blocks, boxes, chunks, dst_sel, src_sel);
+    prolong_kernel<<<dim3(nchunks, 2), XFER_CHUNK, 0, stream>>>(blocks, boxes, chunks, dst_sel, src_sel);
     return cudaGetLastError();
 }
 

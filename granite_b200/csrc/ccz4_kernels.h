@@ -119,12 +119,9 @@ enum GhostMode {
 cudaError_t launch_ghost_fill(int mode, const DevBlock* blocks, const GhostItem* items, int nitems,
                               int sel, const unsigned char* facemask, cudaStream_t stream);
 
-// A box of cells moved between two blocks. Coordinates are block-local cell
-// indices including ghosts.
-//   copy:     dst <- src, same level, cell for cell (s0 = source origin)
-//   prolong:  dst (fine) <- trilinear interpolation of src (coarse), amr.cpp:484-564
-//   restrict: dst (coarse) <- mean of the 2x2x2 fine cells of src at s0 + 2 (a, b, c),
-//             amr.cpp:566-626
+// A box of cells of block dst filled by trilinear interpolation of block src
+// (amr.cpp:484-564). Block-local cell indices including ghosts (s0 is only used
+// on the host).
 struct XferBox {
     int dst, src;
     int d0[3];
@@ -137,11 +134,10 @@ struct BoxChunk {
     int start;
 };
 constexpr int XFER_CHUNK = 256;
-enum XferKind { XFER_COPY = 0, XFER_PROLONG = 1, XFER_RESTRICT = 2 };
 
-// Transfers of slot src_sel of the source blocks into slot dst_sel of the destinations.
-cudaError_t launch_xfer(int kind, const DevBlock* blocks, const XferBox* boxes, const BoxChunk* chunks,
-                        int nchunks, int dst_sel, int src_sel, cudaStream_t stream);
+// Prolongation of slot src_sel of the source blocks into slot dst_sel of the destinations.
+cudaError_t launch_prolong(const DevBlock* blocks, const XferBox* boxes, const BoxChunk* chunks, int nchunks, int dst_sel,
+                           int src_sel, cudaStream_t stream);
 
 // One ghost cell of a level and where its value comes from (GRANITE_AMR_GHOSTS):
 //   src_block >= 0, src_cell >= 0: copy of that cell of a same-level block
@@ -153,9 +149,14 @@ struct GhostSrc {
 
 // Every listed ghost cell written once: copies and local fills read slot
 // `sel`, prolongations read slot 0 of the coarse block. local_mode:
-// GHOST_ZERO_GRADIENT or GHOST_SOMMERFELD.
+// GHOST_ZERO_GRADIENT or GHOST_SOMMERFELD. prolong: prolongated cells are
+// written in this many slots from sel on (0: not at all).
 cudaError_t launch_ghost_sources(const DevBlock* blocks, const GhostSrc* items, long long nitems, int sel,
-                                 int local_mode, cudaStream_t stream);
+                                 int local_mode, int prolong, cudaStream_t stream);
+
+// Restriction of slot 0 (amr.cpp:566-626): every listed coarse cell becomes the
+// mean of the 2x2x2 fine cells of src_block from src_cell on.
+cudaError_t launch_restrict(const DevBlock* blocks, const GhostSrc* items, long long nitems, cudaStream_t stream);
 
 // Constraint monitor (ccz4.cpp:941-1159) over a tile work-list. Writes ham /
 // mom (single-block drop-in; may be null) and per-CTA partial sums of H^2 and
