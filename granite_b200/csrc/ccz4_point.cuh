@@ -108,6 +108,22 @@ __device__ __forceinline__ void ccz4_point(const DevBlock& B, const double* __re
 #pragma unroll
     for (int a = 0; a < 3; ++a) bp[a] = (P)beta[a];
 
+    // the rest of the pointwise state, not needed by the first field loop: loaded
+    // after it, or (Src::UNROLL, few warps to hide a load's latency) before it
+    P At[6], Gh[3], K, Theta, alpha;
+    double alpha_d;
+    auto load_rest = [&]() {
+        alpha_d = __ldg(FP(ALPHA));
+        alpha = (P)alpha_d;
+        K = (P)__ldg(FP(KTR));
+        Theta = (P)__ldg(FP(THETA));
+#pragma unroll
+        for (int a = 0; a < 6; ++a) At[a] = (P)__ldg(FP(AXX + a));
+#pragma unroll
+        for (int a = 0; a < 3; ++a) Gh[a] = (P)__ldg(FP(GHX + a));
+    };
+    if constexpr (Src::UNROLL) load_rest();
+
     // ---- conformal metric: gradients, Hessian term of Ricci, advection ----
     P dg[6][3];     // d_k gt_ij
     P Rt[6];        // conformal Ricci (ccz4.cpp:465-516), accumulated term by term
@@ -148,14 +164,7 @@ __device__ __forceinline__ void ccz4_point(const DevBlock& B, const double* __re
     for (int a = 0; a < 6; ++a)
 #pragma unroll
         for (int d = 0; d < 3; ++d) dg[a][d] = sc[3 * a + d];
-    // the rest of the pointwise state, not needed by the loop above
-    const double alpha_d = __ldg(FP(ALPHA));
-    const P alpha = (P)alpha_d, K = (P)__ldg(FP(KTR)), Theta = (P)__ldg(FP(THETA));
-    P At[6], Gh[3];
-#pragma unroll
-    for (int a = 0; a < 6; ++a) At[a] = (P)__ldg(FP(AXX + a));
-#pragma unroll
-    for (int a = 0; a < 3; ++a) Gh[a] = (P)__ldg(FP(GHX + a));
+    if constexpr (!Src::UNROLL) load_rest();
 
     // first-kind Christoffels G1[k][ij] = 1/2 (d_i g_kj + d_j g_ki - d_k g_ij)
     P G1[3][6];

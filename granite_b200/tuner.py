@@ -1,21 +1,17 @@
 """Autotuner of the TMA stage kernel per block-size class.
 
 The reference evaluates computeRHS with one OpenMP loop per block whatever its
-size (ccz4.cpp:267-270). Here the stage kernel exists in several
-configurations (tile depth, ring depth, shared-memory copies of the stage input
-and of the Hessian-field loop; granite_b200.stage_config_info), and the best one
-depends on the block size (partial tiles along x, halo overhead per tile,
-resident CTAs per SM) and on the precision. For every block-size class (edge
+size (ccz4.cpp:267-270). Here a configuration id chooses the stage kernel's
+tiles (granite_b200.stage_config_info: with x-remainder tiles or without), and
+the better choice depends on the block size and on the precision. For every block-size class (edge
 in STAGE_CLASS_EDGES) and precision this module times every configuration on a
 level of equal cubic blocks of that edge carrying single-puncture data (about
 two million interior points, so a launch takes about a millisecond), with CUDA
 events around every stage launch (the library's profiler), and keeps the
 fastest. The result is a table {"fp64": [cfg per class], "mixed": [...]} that
 Evolver.apply_stage_table applies, and a uniform table (one configuration per
-precision for every class): a level whose blocks use different configurations
-runs one launch per configuration, and on hierarchies of mixed block sizes the
-extra launch tails cost more than the per-class gains, so the library's
-built-in default is the uniform table this module produced on a B200.
+precision for every class). A level whose blocks use different tiles runs one
+launch per tile set; without a table the library chooses one set per level.
 
     python -m granite_b200.tuner [--out table.json] [--classes 16,24] [--configs 0,4] [--precisions mixed]
                                  [--steps 3]
