@@ -604,8 +604,8 @@ cudaError_t copy_out_interior(Ctx* c, double* dst, const double* src, const gran
     const size_t rows = ty * nz;                                 // of a field, from its first interior plane on
     const size_t per_field = (rows + rows_per - 1) / rows_per, pieces = per_field * nv;
     return on_copy_threads(c, pieces, [&](int t, int nt) {
-        size_t first[2], count[2];  // the piece in each slot
-        double* base[2];
+        size_t first[2] = {}, count[2] = {};  // the piece in each slot
+        double* base[2] = {};
         auto finish = [&](int k) {
             cudaError_t e = cudaEventSynchronize(c->pin_ev[2 * t + k]);
             if (e != cudaSuccess) return e;

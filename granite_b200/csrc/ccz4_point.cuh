@@ -81,10 +81,23 @@ __device__ __forceinline__ void ccz4_point(const DevBlock& B, const double* __re
     const double chi_raw = __ldg(FP(CHI));
     const double chi = (isfinite(chi_raw) && chi_raw >= 1.0e-4) ? chi_raw : 1.0e-4;  // :279-280
     double gtd[6], beta[3];
+    // (The global-load kernels walk from field to field with one addition instead
+    // of a product each, 8 % of their time: mixed 89x70x61, 248 us with products,
+    // 229 so. In the TMA kernel, where the pointers would take registers the loops
+    // need, the walk costs FP64 2 %: 471 -> 479 us on 128x128x64.)
+    if constexpr (Src::UNROLL) {
+        const double* q = FP(GXX);
 #pragma unroll
-    for (int a = 0; a < 6; ++a) gtd[a] = __ldg(FP(GXX + a));
+        for (int a = 0; a < 6; ++a, q += st) gtd[a] = __ldg(q);
+        q = FP(BETAX);
 #pragma unroll
-    for (int a = 0; a < 3; ++a) beta[a] = __ldg(FP(BETAX + a));
+        for (int a = 0; a < 3; ++a, q += st) beta[a] = __ldg(q);
+    } else {
+#pragma unroll
+        for (int a = 0; a < 6; ++a) gtd[a] = __ldg(FP(GXX + a));
+#pragma unroll
+        for (int a = 0; a < 3; ++a) beta[a] = __ldg(FP(BETAX + a));
+    }
     // inverse conformal metric, FP64 (ccz4.cpp:318-330)
     double gtud[6];
     {
@@ -113,14 +126,28 @@ __device__ __forceinline__ void ccz4_point(const DevBlock& B, const double* __re
     P At[6], Gh[3], K, Theta, alpha;
     double alpha_d;
     auto load_rest = [&]() {
-        alpha_d = __ldg(FP(ALPHA));
+        if constexpr (Src::UNROLL) {
+            static_assert(KTR == AXX + 6 && GHX == KTR + 1 && THETA == GHX + 3 && ALPHA == THETA + 1, "in a row");
+            const double* q = FP(AXX);
+#pragma unroll
+            for (int a = 0; a < 6; ++a, q += st) At[a] = (P)__ldg(q);
+            K = (P)__ldg(q);
+            q += st;
+#pragma unroll
+            for (int a = 0; a < 3; ++a, q += st) Gh[a] = (P)__ldg(q);
+            Theta = (P)__ldg(q);
+            q += st;
+            alpha_d = __ldg(q);
+        } else {
+            alpha_d = __ldg(FP(ALPHA));
+            K = (P)__ldg(FP(KTR));
+            Theta = (P)__ldg(FP(THETA));
+#pragma unroll
+            for (int a = 0; a < 6; ++a) At[a] = (P)__ldg(FP(AXX + a));
+#pragma unroll
+            for (int a = 0; a < 3; ++a) Gh[a] = (P)__ldg(FP(GHX + a));
+        }
         alpha = (P)alpha_d;
-        K = (P)__ldg(FP(KTR));
-        Theta = (P)__ldg(FP(THETA));
-#pragma unroll
-        for (int a = 0; a < 6; ++a) At[a] = (P)__ldg(FP(AXX + a));
-#pragma unroll
-        for (int a = 0; a < 3; ++a) Gh[a] = (P)__ldg(FP(GHX + a));
     };
     if constexpr (Src::UNROLL) load_rest();
 
