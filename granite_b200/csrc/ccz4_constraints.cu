@@ -23,16 +23,23 @@ __device__ void constraint_point(const DevBlock& B, const double* __restrict__ u
     const long long st = B.stride;
     const double* __restrict__ uc = u + c;
 #define FP(v) (uc + (long long)(v) * st)
-    const double chi = __ldg(FP(CHI));
-    const double K = __ldg(FP(KTR));
+    // Pointers walk from field to field (one addition instead of a product each):
+    // with the int neighbour offsets the monitor of 128^3 takes 486 us instead of
+    // 529. What bounds it is the latency of its loads at 8 warps per SM (255
+    // registers; three CTAs per SM spill and are slower).
+    static_assert(CHI == 0 && GXX == 1 && AXX == GXX + 6 && KTR == AXX + 6 && GHX == KTR + 1, "in a row");
     double gt[6], At[6], Gh[3], gtu[6];
+    const double* q = uc;
+    const double chi = __ldg(q);
+    q += st;
 #pragma unroll
-    for (int a = 0; a < 6; ++a) {
-        gt[a] = __ldg(FP(GXX + a));
-        At[a] = __ldg(FP(AXX + a));
-    }
+    for (int a = 0; a < 6; ++a, q += st) gt[a] = __ldg(q);
 #pragma unroll
-    for (int a = 0; a < 3; ++a) Gh[a] = __ldg(FP(GHX + a));
+    for (int a = 0; a < 6; ++a, q += st) At[a] = __ldg(q);
+    const double K = __ldg(q);
+    q += st;
+#pragma unroll
+    for (int a = 0; a < 3; ++a, q += st) Gh[a] = __ldg(q);
     {
         const double det = gt[0] * (gt[3] * gt[5] - gt[4] * gt[4]) - gt[1] * (gt[1] * gt[5] - gt[4] * gt[2]) +
             gt[2] * (gt[1] * gt[4] - gt[3] * gt[2]);
@@ -46,9 +53,10 @@ __device__ void constraint_point(const DevBlock& B, const double* __restrict__ u
     }
     const double beta0[3] = {0.0, 0.0, 0.0};
     double dg[6][3], Rt[6];
+    q = FP(GXX);
 #pragma unroll
-    for (int a = 0; a < 6; ++a) {
-        FieldDer<P> fd = field_der_noko<P, true>(B, FP(GXX + a), beta0, 0.0);
+    for (int a = 0; a < 6; ++a, q += st) {
+        FieldDer<P> fd = field_der_noko<P, true>(B, q, beta0, 0.0);
 #pragma unroll
         for (int d = 0; d < 3; ++d) dg[a][d] = fd.d[d];
         Rt[a] = -0.5 * (gtu[0] * fd.h[0] + gtu[3] * fd.h[3] + gtu[5] * fd.h[5] +
@@ -72,9 +80,10 @@ __device__ void constraint_point(const DevBlock& B, const double* __restrict__ u
         Gc[k] = gtu[0] * ch[k][0] + gtu[3] * ch[k][3] + gtu[5] * ch[k][5] +
             2.0 * (gtu[1] * ch[k][1] + gtu[2] * ch[k][2] + gtu[4] * ch[k][4]);
     double dGh[3][3];
+    q = FP(GHX);
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        FieldDer<P> fd = field_der_noko<P, false>(B, FP(GHX + a), beta0, 0.0);
+    for (int a = 0; a < 3; ++a, q += st) {
+        FieldDer<P> fd = field_der_noko<P, false>(B, q, beta0, 0.0);
 #pragma unroll
         for (int d = 0; d < 3; ++d) dGh[a][d] = fd.d[d];
     }
@@ -146,14 +155,15 @@ __device__ void constraint_point(const DevBlock& B, const double* __restrict__ u
 
     // momentum constraint, ccz4.cpp:1138-1155
     double dA[6][3], dK[3];
+    q = FP(AXX);
 #pragma unroll
-    for (int a = 0; a < 6; ++a) {
-        FieldDer<P> fd = field_der_noko<P, false>(B, FP(AXX + a), beta0, 0.0);
+    for (int a = 0; a < 6; ++a, q += st) {
+        FieldDer<P> fd = field_der_noko<P, false>(B, q, beta0, 0.0);
 #pragma unroll
         for (int d = 0; d < 3; ++d) dA[a][d] = fd.d[d];
     }
     {
-        FieldDer<P> fd = field_der_noko<P, false>(B, FP(KTR), beta0, 0.0);
+        FieldDer<P> fd = field_der_noko<P, false>(B, q, beta0, 0.0);
 #pragma unroll
         for (int d = 0; d < 3; ++d) dK[d] = fd.d[d];
     }

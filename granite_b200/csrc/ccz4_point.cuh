@@ -63,7 +63,7 @@ struct GlobalSource {
     template <bool HESS, bool EXACT, bool KOSEP, typename P>
     __device__ __forceinline__ FieldDer<P> der(int v, const Advection<P, EXACT>& adv) {
         return field_der_l<P, HESS, true, EXACT, KOSEP>(
-            B, GlobalLoad{u + (long long)v * B.stride + c, {1, B.tx, (long long)B.tx * B.ty}}, adv);
+            B, global_load<EXACT>(u + (long long)v * B.stride + c, B.tx, B.ty), adv);
     }
 };
 

@@ -16,6 +16,8 @@
 //    FP32 without losing the cancellation.
 #pragma once
 
+#include <type_traits>
+
 #include "ccz4_common.cuh"
 
 namespace granite_b200 {
@@ -39,16 +41,27 @@ struct StridedAxis {
 // Stencil loaders of one field at one point: operator()(o) is the value o cells
 // away in the field's storage, stride(d) the cell offset along axis d, and
 // axis<D>(beta) the neighbours along axis D.
+// Offsets in int where every stencil is FP64 (EXACT): one wide multiply-add per
+// neighbour instead of a 64-bit addition chain, 4 % of the FP64 global-load RHS
+// (89x70x61: 335 -> 322 us); the mixed build's pair stencils are 8 % slower so
+// (234 -> 253 us) and keep 64-bit offsets. Four planes of cells always fit an
+// int: 2^29 cells in one plane are 850 GB for a block's nine planes or more.
+template <typename O>
 struct GlobalLoad {  // read-only global memory through the non-coherent path
     const double* __restrict__ p;
-    long long off[3];
-    __device__ __forceinline__ double operator()(long long o) const { return __ldg(p + o); }
-    __device__ __forceinline__ long long stride(int d) const { return off[d]; }
+    O off[3];
+    __device__ __forceinline__ double operator()(O o) const { return __ldg(p + o); }
+    __device__ __forceinline__ O stride(int d) const { return off[d]; }
     template <int D>
-    __device__ __forceinline__ StridedAxis<GlobalLoad, long long> axis(double beta) const {
+    __device__ __forceinline__ StridedAxis<GlobalLoad, O> axis(double beta) const {
         return {*this, off[D], beta >= 0.0 ? -4 * off[D] : 4 * off[D]};
     }
 };
+template <bool EXACT>
+__device__ __forceinline__ auto global_load(const double* f, int tx, int ty) {
+    using O = std::conditional_t<EXACT, int, long long>;
+    return GlobalLoad<O>{f, {1, tx, (O)tx * ty}};
+}
 template <int SY, int SZ>
 struct SharedLoad {  // a CTA-staged tile in shared memory, rows of SY and planes of SZ cells
     const double* p;
@@ -312,7 +325,7 @@ __device__ __forceinline__ FieldDer<P> field_der_l(const StencilCoef& B, const L
 template <typename P, bool HESS>
 __device__ __forceinline__ FieldDer<P> field_der_noko(const DevBlock& B, const double* __restrict__ f,
                                                       const double beta[3], P w) {
-    return field_der_l<P, HESS, false, true>(B, GlobalLoad{f, {1, B.tx, (long long)B.tx * B.ty}},
+    return field_der_l<P, HESS, false, true>(B, global_load<true>(f, B.tx, B.ty),
                                              Advection<P, true>(B, beta, w));
 }
 
