@@ -35,9 +35,9 @@
 //
 // Every wait is bounded (TMA_WAIT_NS): a thread whose wait gives up records it
 // in StageArgs::errflag and skips its later waits; a compute warp then leaves
-// after its current tile, and a load warp stops issuing, waits (bounded) for
-// the copies it issued and leaves, so the kernel always ends and no copy into
-// shared memory outlives the CTA.
+// at its next tile, and the load warp stops issuing, waits (bounded) for the
+// copies it issued and leaves, so the kernel always ends and no copy into shared
+// memory outlives the CTA.
 #pragma once
 
 #include <cstdint>
@@ -80,6 +80,9 @@ __device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
 __device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(unsigned bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
+}
 __device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity) {
     unsigned ok;
     asm volatile(
@@ -103,10 +106,17 @@ __device__ __forceinline__ void tma_load_box(unsigned dst, const void* map, int 
         "l"(map), "r"(x), "r"(y), "r"(z), "r"(f), "r"(bar)
         : "memory");
 }
-// Wait limit of one ring slot: 2 s of wall time, then the kernel records the
-// failure in StageArgs::errflag and stops waiting (results are then garbage
-// and the host reports the error).
-constexpr unsigned long long TMA_WAIT_NS = 2000000000ull;
+
+}  // namespace
+
+}  // namespace granite_b200
+
+#include "ccz4_stage_ring.cuh"
+
+namespace granite_b200 {
+
+namespace {
+
 // NWG compute warpgroups, NBUF ring slots each; REM: x-remainder tiles
 // (TMA_REM_X x 4 x 4 points, slots sized for their boxes).
 template <int NWG_, int NBUF_, bool REM_>
@@ -130,67 +140,19 @@ struct TmaKernelT {
     static_assert(COMP_REGS <= 255 && COMP_REGS >= 128, "compute warps");
 };
 
-__device__ __forceinline__ void mbar_arrive(unsigned bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
-}
-// Bounded wait for the completion of the phase of parity `parity`; on a timeout
-// the failure is recorded. Returns false then. A waiting warp is suspended
-// within each attempt (mbarrier.try_wait); the clock is read every 64 of them.
-__device__ __forceinline__ bool tma_wait(unsigned bar, unsigned parity, unsigned int* err) {
-    if (mbar_try_wait(bar, parity)) return true;
-    unsigned long long t0 = 0;
-#pragma unroll 1
-    for (unsigned n = 0;; ++n) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (n % 64 == 0) {
-            const unsigned long long t = global_ns();
-            if (n == 0) t0 = t;
-            if (t - t0 > TMA_WAIT_NS) {
-                if (err) atomicExch(err, 1u);
-                return false;
-            }
-        }
-    }
-}
-
-// Tile of a compute warpgroup's round r at [r & 1] (index < 0: no more tiles)
-// and its block's descriptor.
-struct __align__(16) TmaTile {
-    Tile t;
-    int index;
-    int pad[2];
-};
-constexpr int TMA_MAX_SLOTS = 4;
-struct TmaShared {
-    unsigned long long full[TMA_MAX_SLOTS], empty[TMA_MAX_SLOTS];
-    TmaTile tile[2];
-    __align__(16) unsigned char block[2][sizeof(DevBlock)];
-};
-static_assert(sizeof(Tile) == 5 * sizeof(int) && sizeof(DevBlock) % 8 == 0 && sizeof(DevBlock) / 8 <= 64,
-              "copied by one warp: a word of the tile and two words of the descriptor per lane");
-__shared__ TmaShared g_tma[4];
-
 // The compute warps' stencil source.
 template <class C, bool UC>
 struct TmaSource {
     static constexpr bool UNROLL = false;
-    unsigned ring0;  // shared address of the ring
-    const TmaShared& sh;
-    unsigned full0, empty0;
+    unsigned slots;  // shared address of the ring's slots
+    TmaRing<C::NBUF> ring;
     const StencilCoef& coef;  // UC: the coefficients of every block of the launch, in the kernel arguments
-    unsigned int* err;
     int lin = 0;
     ArmOffsets arm{};
     int round = 0;
-    int slot = 0;        // ring slot of the next field
-    unsigned phase = 0;  // and the parity of its phase
-    bool failed = false;
 
     __device__ __forceinline__ const DevBlock& block() const {
-        return *reinterpret_cast<const DevBlock*>(sh.block[round & 1]);
-    }
-    __device__ __forceinline__ void wait() {
-        if (!failed) failed = !tma_wait(full0 + 8u * slot, phase, err);
+        return *reinterpret_cast<const DevBlock*>(ring.sh.block[round & 1]);
     }
     __device__ __forceinline__ const StencilCoef& coefs() const {
         if constexpr (UC)
@@ -200,127 +162,14 @@ struct TmaSource {
     }
     template <bool HESS, bool EXACT, bool KOSEP, typename P>
     __device__ __forceinline__ FieldDer<P> der(int /*v*/, const Advection<P, EXACT>& adv) {
-        wait();
-        const unsigned at = ring0 + slot * (unsigned)(C::SLOT * sizeof(double));
+        ring.wait();
+        const unsigned at = slots + ring.slot * (unsigned)(C::SLOT * sizeof(double));
         const SplitLoad<C::BX, C::BX * C::BY> L{at, at + lin, arm};
         const FieldDer<P> r = field_der_l<P, HESS, true, EXACT, KOSEP>(coefs(), L, adv);
-        // every lane's loads of the slot come before the warp's arrival
-        __syncwarp();
-        if ((threadIdx.x & 31) == 0) mbar_arrive(empty0 + 8u * slot);
-        if (++slot == C::NBUF) slot = 0, phase ^= 1u;
+        ring.release();
         return r;
     }
 };
-
-// The tiles of one compute warpgroup in order: list entries first, first +
-// stride, ..., or with SEL those of them whose flag is `want`. Warp-wide.
-template <bool SEL>
-struct TmaTileFinder {
-    const unsigned char* flags;
-    int want, ntiles, stride;
-    int next;              // next list entry to look at
-    int base = 0;          // SEL: entry of lane 0 of the last 32 looked at
-    unsigned pending = 0;  // and those of them still to be taken
-    __device__ __forceinline__ int find() {
-        if constexpr (SEL) {
-            while (!pending) {
-                if (next >= ntiles) return -1;
-                base = next;
-                const long long ti = base + (long long)(threadIdx.x & 31) * stride;
-                pending = __ballot_sync(0xffffffffu, ti < ntiles && flags[ti] == want);
-                next = (int)min((long long)ntiles, base + 32ll * stride);
-            }
-            const int b = __ffs(pending) - 1;
-            pending &= pending - 1;
-            return base + b * stride;
-        } else {
-            const int t = next;
-            if (t >= ntiles) return -1;
-            next = ntiles - t > stride ? t + stride : ntiles;
-            return t;
-        }
-    }
-};
-
-// One load warp: every lane takes part in the tile search, the copies of tile
-// and descriptor and the waits; lane 0 issues the box loads.
-template <class C, bool SEL>
-__device__ __forceinline__ void tma_load_warp(int g, const DevBlock* __restrict__ blocks, const Tile* __restrict__ tiles,
-                                             int ntiles, const StageArgs& A, unsigned ring0) {
-    TmaShared& sh = g_tma[g];
-    const int lane = threadIdx.x & 31;
-    const unsigned full0 = smem_addr(sh.full), empty0 = smem_addr(sh.empty);
-    constexpr int WORDS = sizeof(DevBlock) / 8;
-    TmaTileFinder<SEL> finder{A.tile_prec, A.want_prec, ntiles, (int)gridDim.x * C::NWG,
-                             (int)(g * gridDim.x + blockIdx.x)};
-    // the tile of the coming round: its list entry, this lane's word of it and this lane's words of the descriptor
-    int ti = finder.find();
-    int tw = ti >= 0 && lane < 5 ? reinterpret_cast<const int*>(tiles + ti)[lane] : 0;
-    unsigned long long d0 = 0, d1 = 0;
-    auto load_desc = [&](int word, unsigned long long& x0, unsigned long long& x1) {
-        const unsigned long long* src =
-            reinterpret_cast<const unsigned long long*>(blocks + __shfl_sync(0xffffffffu, word, 0));
-        x0 = src[lane];
-        if (lane + 32 < WORDS) x1 = src[lane + 32];
-    };
-    if (ti >= 0) load_desc(tw, d0, d1);
-    int slot = 0, q = 0;
-    unsigned ephase = 1;               // parity of the slot's empty phase: the first pass finds the slots empty
-    unsigned issued = 0, parity = 0;   // per slot: a copy was issued into it; the phases its barrier will complete, mod 2
-    bool ok = true;
-    for (int r = 0; ok; ++r) {
-        // (all compute warps have left round r - 2: each arrived on a field of round r - 1)
-        TmaTile& T = sh.tile[r & 1];
-        if (lane < 5) reinterpret_cast<int*>(&T.t)[lane] = tw;
-        if (lane == 5) T.index = ti;
-        unsigned long long* B = reinterpret_cast<unsigned long long*>(sh.block[r & 1]);
-        B[lane] = d0;
-        if (lane + 32 < WORDS) B[lane + 32] = d1;
-        __syncwarp();
-        if (ti < 0) {  // no more tiles: the compute warps see it behind the next slot's barrier
-            if ((ok = tma_wait(empty0 + 8u * slot, ephase, A.errflag)) && lane == 0) {
-                mbar_arrive(full0 + 8u * slot);
-                parity ^= 1u << slot;  // the slot's barrier completes one phase more than its copies
-            }
-            break;
-        }
-        const int blk = __shfl_sync(0xffffffffu, tw, 0), i0 = __shfl_sync(0xffffffffu, tw, 1),
-                  j0 = __shfl_sync(0xffffffffu, tw, 2), k0 = __shfl_sync(0xffffffffu, tw, 3);
-        const bool rem = C::REM && __shfl_sync(0xffffffffu, tw, 4) < 0;
-        const size_t map = (size_t)(3 * blk + A.in_sel) * 128;
-        const unsigned char* m = static_cast<const unsigned char*>(rem ? A.tmaps_rem : A.tmaps) + map;
-        const unsigned char* ma = static_cast<const unsigned char*>(A.tmaps_arm) + map;
-        const int zhi = k0 + (rem ? 2 * C::TZ : C::TZ) + 5;
-        constexpr unsigned ARM = C::Boxes::ARM * sizeof(double);
-        const unsigned arm = (rem ? C::BoxesRem::MAIN : C::Boxes::MAIN) * (unsigned)sizeof(double);
-        const unsigned bytes = (rem ? C::BoxesRem::CELLS : C::Boxes::CELLS) * (unsigned)sizeof(double);
-        ti = finder.find();
-        tw = ti >= 0 && lane < 5 ? reinterpret_cast<const int*>(tiles + ti)[lane] : 0;
-        for (int p = 0; p < NV; ++p) {
-            if (!(ok = tma_wait(empty0 + 8u * slot, ephase, A.errflag))) break;
-            // test switch: item test_withhold - 1 of the first warpgroup is never issued
-            if (lane == 0 && !(A.test_withhold != 0 && q == A.test_withhold - 1 && blockIdx.x == 0 && g == 0)) {
-                const unsigned bar = full0 + 8u * slot, dst = ring0 + slot * (unsigned)(C::SLOT * sizeof(double));
-                const int f = FIELD_ORDER[p];
-                mbar_expect_tx(bar, bytes);
-                // (an interior index is also the cell, incl. ghosts, four lower)
-                tma_load_box(dst, m, i0, j0, k0 + 3, f, bar);
-                tma_load_box(dst + arm, ma, i0 + NG, j0 + NG, k0, f, bar);
-                tma_load_box(dst + arm + ARM, ma, i0 + NG, j0 + NG, zhi, f, bar);
-                issued |= 1u << slot;
-                parity ^= 1u << slot;
-            }
-            __syncwarp();
-            if (++slot == C::NBUF) slot = 0, ephase ^= 1u;
-            ++q;
-            if (p == NV / 2 && ti >= 0) load_desc(tw, d0, d1);
-        }
-    }
-    // no copy into shared memory outlives the CTA: wait for the last one of every slot
-    if (lane == 0)
-        for (int s = 0; s < C::NBUF; ++s)
-            if (issued >> s & 1u) tma_wait(full0 + 8u * s, (parity >> s & 1u) ^ 1u, A.errflag);
-}
 
 }  // namespace
 
@@ -330,11 +179,13 @@ __global__ void __launch_bounds__(C::NTHR, 1)
                          const __grid_constant__ StageArgs A) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int g = threadIdx.x / C::NP;  // warpgroup
-    if (threadIdx.x < C::NWG)
+    if (threadIdx.x < C::NWG) {
+        g_tma[threadIdx.x].stop = 0;
         for (int s = 0; s < C::NBUF; ++s) {
             mbar_init(smem_addr(&g_tma[threadIdx.x].full[s]), 1);
             mbar_init(smem_addr(&g_tma[threadIdx.x].empty[s]), C::NP / 32);  // every compute warp arrives
         }
+    }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     __syncthreads();
     const unsigned rings = smem_addr(smem_raw);
@@ -348,11 +199,10 @@ __global__ void __launch_bounds__(C::NTHR, 1)
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(C::COMP_REGS));
     const int pt = threadIdx.x % C::NP;
     TmaShared& sh = g_tma[g];
-    TmaSource<C, UC> S{rings + g * RING, sh, smem_addr(sh.full), smem_addr(sh.empty), A.coef, A.errflag};
+    TmaSource<C, UC> S{rings + g * RING, {sh, smem_addr(sh.full), smem_addr(sh.empty), A.errflag}, A.coef};
 #pragma unroll 1
     for (int r = 0;; ++r) {
-        S.wait();  // the round's first field, and with it the tile and its descriptor
-        if (S.failed) break;
+        if (!S.ring.next_round()) break;
         const Tile t = sh.tile[r & 1].t;
         const int ti = sh.tile[r & 1].index;
         if (ti < 0) break;
@@ -381,7 +231,6 @@ __global__ void __launch_bounds__(C::NTHR, 1)
         point_pm<PM>(B, B.buf[A.in_sel], c, A, S, L);
         const int2 pr = A.push ? A.tile_push[ti] : make_int2(0, 0);
         if (valid) stage_epilogue<EPI>(B, A, c, L, A.push ? A.push + pr.x : nullptr, pr.y, i, j, k);
-        if (S.failed) break;
     }
 }
 

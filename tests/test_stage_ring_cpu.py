@@ -1,0 +1,29 @@
+"""The stage kernel's ring protocol on host threads (tests/cpp/test_stage_ring.cpp):
+load warp and compute warps with waits that run out in some lanes only."""
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CXX = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
+
+
+@pytest.fixture(scope="module")
+def exe(tmp_path_factory):
+    out = tmp_path_factory.mktemp("ring") / "test_stage_ring"
+    cpp = os.path.join(ROOT, "tests", "cpp")
+    subprocess.run([CXX, "-std=c++17", "-O1", "-pthread", "-I", os.path.join(cpp, "host_cuda"),
+                    "-I", os.path.join(ROOT, "granite_b200", "csrc"), os.path.join(cpp, "test_stage_ring.cpp"),
+                    "-o", str(out)], check=True)
+    return str(out)
+
+
+@pytest.mark.parametrize("what", ["tiles", "selected", "load_lane_late 0", "load_lane_late 9", "compute_lane_late 0",
+                                  "compute_lane_late 13",
+                                  # the run has 154 items: one in its midst, and those before the end of the list
+                                  "compute_warps_late 28", "compute_warps_late 151", "compute_warps_late 153"])
+def test_ring(exe, what):
+    r = subprocess.run([exe, *what.split()], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
+    assert r.stdout.strip() == "OK"
