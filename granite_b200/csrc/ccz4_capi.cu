@@ -652,7 +652,7 @@ int stage_single(Ctx* c, const granite_block_desc* b, double* u_dev, int* ntiles
     d.buf[0] = u_dev ? u_dev : c->s_u;
     if (variant == VARIANT_TMA) {
         CUtensorMap m[2];
-        if (encode_block_tmap(&m[0], d.buf[0], d, 0) && encode_block_tmap(&m[1], d.buf[0], d, TMA_SHAPE_ARM))
+        if (tma_available() && encode_block_tmap(&m[0], d.buf[0], d, 0) && encode_block_tmap(&m[1], d.buf[0], d, TMA_SHAPE_ARM))
             CK(cudaMemcpyAsync(c->s_tmap, m, sizeof(m), cudaMemcpyHostToDevice, s), "upload tensor maps");
         else
             variant = VARIANT_GLOBAL;
@@ -1342,7 +1342,7 @@ static int build_lists(Ctx* c) {
     if (c->variant == VARIANT_TMA) {
         std::vector<CUtensorMap> maps(TMA_SHAPES * 3 * nb);
         for (size_t i = 0; i < nb; ++i) {
-            bool ok = true;
+            bool ok = tma_available();
             for (int sh = 0; sh < TMA_SHAPES && ok; ++sh)
                 for (int sl = 0; sl < 3; ++sl)
                     ok = ok && encode_block_tmap(&maps[(sh * nb + i) * 3 + sl], c->hblocks[i].buf[sl], c->hblocks[i], sh);

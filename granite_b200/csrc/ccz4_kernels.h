@@ -78,6 +78,10 @@ bool encode_block_tmap(void* map128, const double* base, const DevBlock& d, int 
 // Per-device kernel attributes (shared-memory opt-in); call with the device current.
 cudaError_t configure_stage_kernels();
 
+// Whether every kernel of the TMA variant may be launched on the current device
+// (TmaGrids); without, its blocks use the global-load kernel.
+bool tma_available();
+
 // Precision modes of the stage kernels: FP64 algebra with the reference-order
 // FP64 stencils, FP32 algebra (mixed), or FP64 algebra with pair-difference
 // FP64 stencils (PM_FP64F, RK epilogue only: the FP64 pass of the per-tile

@@ -21,6 +21,7 @@
 #include "ccz4_kernels.h"
 #include "ccz4_point.cuh"
 #include "ccz4_stencil.cuh"
+#include "ccz4_tma_grids.h"
 
 namespace granite_b200 {
 
@@ -256,11 +257,11 @@ static cudaError_t configure_smem() {
 }
 
 // The tile sets of the TMA kernel, one translation unit each (ccz4_tma_tiles<k>.cu).
-using TmaConfigure = cudaError_t (*)(int nsm, int grids[3][2][2]);
+using TmaConfigure = cudaError_t (*)(int nsm, TmaGrids& grids);
 using TmaLaunch = cudaError_t (*)(int pm, int epi, bool sel, const DevBlock* blocks, const Tile* tiles, int ntiles,
                                   const StageArgs& args, cudaStream_t stream, int grid);
-cudaError_t configure_tma_tiles0(int, int[3][2][2]);
-cudaError_t configure_tma_tiles1(int, int[3][2][2]);
+cudaError_t configure_tma_tiles0(int, TmaGrids&);
+cudaError_t configure_tma_tiles1(int, TmaGrids&);
 cudaError_t launch_tma_tiles0(int, int, bool, const DevBlock*, const Tile*, int, const StageArgs&, cudaStream_t, int);
 cudaError_t launch_tma_tiles1(int, int, bool, const DevBlock*, const Tile*, int, const StageArgs&, cudaStream_t, int);
 static const TmaConfigure g_tma_configure[NUM_TMA_TILESETS] = {configure_tma_tiles0, configure_tma_tiles1};
@@ -268,7 +269,7 @@ static const TmaLaunch g_tma_launch[NUM_TMA_TILESETS] = {launch_tma_tiles0, laun
 
 // Persistent grid of each TMA kernel on each device (one CTA per SM).
 constexpr int MAX_DEVICES = 64;
-static int g_tma_grid[MAX_DEVICES][NUM_TMA_TILESETS][3][2][2];  // [device][tile set][precision mode][epi][sel]
+static TmaGrids g_tma_grid[MAX_DEVICES][NUM_TMA_TILESETS];
 
 static cudaError_t launch_tma(int tileset, int pm, int epi, const DevBlock* blocks, const Tile* tiles, int ntiles,
                               const StageArgs& args, cudaStream_t stream) {
@@ -279,9 +280,17 @@ static cudaError_t launch_tma(int tileset, int pm, int epi, const DevBlock* bloc
     if (e != cudaSuccess) return e;
     const bool sel = args.tile_prec != nullptr;  // per-tile precision passes (RK epilogue)
     if (sel && epi != EPI_RK) return cudaErrorInvalidValue;
-    const int cap = (dev >= 0 && dev < MAX_DEVICES) ? g_tma_grid[dev][tileset][pm][epi][sel ? 1 : 0] : 0;
+    const int cap = (dev >= 0 && dev < MAX_DEVICES) ? g_tma_grid[dev][tileset].of(pm, epi, sel, args.coef_uniform != 0) : 0;
     if (cap <= 0) return cudaErrorInvalidConfiguration;  // not instantiated, or configure_stage_kernels() not run
     return g_tma_launch[tileset](pm, epi, sel, blocks, tiles, ntiles, args, stream, ntiles < cap ? ntiles : cap);
+}
+
+bool tma_available() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return false;
+    for (const TmaGrids& g : g_tma_grid[dev])
+        if (g.refused) return false;
+    return true;
 }
 
 // Opt the shared-memory variants into more than 48 KB of dynamic shared memory

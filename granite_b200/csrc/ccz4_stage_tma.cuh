@@ -44,6 +44,7 @@
 #include <type_traits>
 
 #include "ccz4_point.cuh"
+#include "ccz4_tma_grids.h"
 
 namespace granite_b200 {
 
@@ -235,21 +236,21 @@ __global__ void __launch_bounds__(C::NTHR, 1)
 }
 
 // Launchers of one tile set: C3 the mixed kernels (12 compute warps per SM), C2
-// the FP64 ones (8). grids[pm][epi][sel]: the persistent grid, 0 = not instantiated.
+// the FP64 ones (8).
 template <class C3, class C2>
 struct TmaKernelOps {
     template <int PM>
     using Cfg = typename std::conditional<PM == PM_MIXED, C3, C2>::type;
     // the register split needs the launch's full share: setmaxnreg.inc would wait for registers that never free up
     template <int PM, int EPI, bool SEL, bool UC>
-    static cudaError_t configure_one(int nsm, int grids[3][2][2]) {
+    static cudaError_t configure_one(int nsm, TmaGrids& grids) {
         using C = Cfg<PM>;
         auto k = ccz4_stage_tma_kernel<PM, EPI, C, SEL, UC>;
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
         if (e != cudaSuccess) return e;
         cudaFuncAttributes fa{};
         if ((e = cudaFuncGetAttributes(&fa, k))) return e;
-        grids[PM][EPI][SEL ? 1 : 0] = fa.numRegs == C::LAUNCH_REGS ? nsm : 0;  // 0: not available
+        grids.put(PM, EPI, SEL, UC, fa.numRegs, C::LAUNCH_REGS, nsm);
         return cudaSuccess;
     }
     template <int PM, int EPI, bool SEL, bool UC>
@@ -260,7 +261,7 @@ struct TmaKernelOps {
         return cudaGetLastError();
     }
     template <bool UC>
-    static cudaError_t configure_rk(int nsm, int grids[3][2][2]) {
+    static cudaError_t configure_rk(int nsm, TmaGrids& grids) {
         cudaError_t e;
         if ((e = configure_one<PM_FP64, EPI_RK, false, UC>(nsm, grids))) return e;
         if ((e = configure_one<PM_MIXED, EPI_RK, false, UC>(nsm, grids))) return e;
@@ -278,7 +279,7 @@ struct TmaKernelOps {
     }
     // STORE: plus the store epilogue (single-block launches, always uniform).
     template <bool STORE>
-    static cudaError_t configure(int nsm, int grids[3][2][2]) {
+    static cudaError_t configure(int nsm, TmaGrids& grids) {
         cudaError_t e;
         if ((e = configure_rk<false>(nsm, grids))) return e;
         if ((e = configure_rk<true>(nsm, grids))) return e;

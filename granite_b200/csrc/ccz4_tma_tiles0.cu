@@ -7,7 +7,7 @@
 
 namespace granite_b200 {
 using Ops0 = TmaKernelOps<TmaKernelT<3, 3, false>, TmaKernelT<2, 4, false>>;
-cudaError_t configure_tma_tiles0(int nsm, int grids[3][2][2]) { return Ops0::configure<true>(nsm, grids); }
+cudaError_t configure_tma_tiles0(int nsm, TmaGrids& grids) { return Ops0::configure<true>(nsm, grids); }
 cudaError_t launch_tma_tiles0(int pm, int epi, bool sel, const DevBlock* blocks, const Tile* tiles, int ntiles,
                               const StageArgs& args, cudaStream_t stream, int grid) {
     return Ops0::launch<true>(pm, epi, sel, blocks, tiles, ntiles, args, stream, grid);

@@ -7,7 +7,7 @@
 
 namespace granite_b200 {
 using Ops1 = TmaKernelOps<TmaKernelT<3, 3, true>, TmaKernelT<2, 4, true>>;
-cudaError_t configure_tma_tiles1(int nsm, int grids[3][2][2]) { return Ops1::configure<false>(nsm, grids); }
+cudaError_t configure_tma_tiles1(int nsm, TmaGrids& grids) { return Ops1::configure<false>(nsm, grids); }
 cudaError_t launch_tma_tiles1(int pm, int epi, bool sel, const DevBlock* blocks, const Tile* tiles, int ntiles,
                               const StageArgs& args, cudaStream_t stream, int grid) {
     return Ops1::launch<false>(pm, epi, sel, blocks, tiles, ntiles, args, stream, grid);

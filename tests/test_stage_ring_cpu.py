@@ -1,5 +1,6 @@
-"""The stage kernel's ring protocol on host threads (tests/cpp/test_stage_ring.cpp):
-load warp and compute warps with waits that run out in some lanes only."""
+"""Host parts of the stage kernel without a device: its ring protocol on host threads
+(tests/cpp/test_stage_ring.cpp: load warp and compute warps with waits that run
+out in some lanes only) and the table of kernels that may be launched."""
 import os
 import subprocess
 
@@ -9,14 +10,17 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CXX = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
 
 
-@pytest.fixture(scope="module")
-def exe(tmp_path_factory):
-    out = tmp_path_factory.mktemp("ring") / "test_stage_ring"
+def build(out, name):
     cpp = os.path.join(ROOT, "tests", "cpp")
     subprocess.run([CXX, "-std=c++17", "-O1", "-pthread", "-I", os.path.join(cpp, "host_cuda"),
-                    "-I", os.path.join(ROOT, "granite_b200", "csrc"), os.path.join(cpp, "test_stage_ring.cpp"),
-                    "-o", str(out)], check=True)
-    return str(out)
+                    "-I", os.path.join(ROOT, "granite_b200", "csrc"), os.path.join(cpp, name + ".cpp"),
+                    "-o", str(out / name)], check=True)
+    return str(out / name)
+
+
+@pytest.fixture(scope="module")
+def exe(tmp_path_factory):
+    return build(tmp_path_factory.mktemp("ring"), "test_stage_ring")
 
 
 @pytest.mark.parametrize("what", ["tiles", "selected", "load_lane_late 0", "load_lane_late 9", "compute_lane_late 0",
@@ -27,3 +31,8 @@ def test_ring(exe, what):
     r = subprocess.run([exe, *what.split()], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
     assert r.stdout.strip() == "OK"
+
+
+def test_every_kernel_answers_for_its_registers(tmp_path):
+    r = subprocess.run([build(tmp_path, "test_tma_grids")], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout + r.stderr
