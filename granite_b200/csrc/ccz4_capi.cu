@@ -266,6 +266,11 @@ struct Ctx {
     double* s_partials = nullptr;
     int s_partials_cap = 0;
     double* s_sum = nullptr;
+    // the last launch that reads s_desc, s_tiles and s_tmap: its stream's id (0: none
+    // yet) and, unless that is the context's own stream, an event behind it
+    unsigned long long s_stream = 0;
+    bool s_on_own = false;
+    cudaEvent_t s_done = nullptr;
 
     // pinned staging slots of the host-buffer copy at hand, two per copy thread,
     // each with the event of its last copy; pin_own: this context's own set
@@ -641,6 +646,34 @@ cudaError_t copy_out_interior(Ctx* c, double* dst, const double* src, const gran
     });
 }
 
+// A call on another stream than the last one's lets the last launch finish before
+// it overwrites what that launch reads (the kernel reads its tiles and
+// descriptors to its end). Streams under capture are left out, as an event of
+// work outside the capture cannot be waited for inside it.
+cudaError_t stateless_begin(Ctx* c, cudaStream_t s) {
+    unsigned long long id = 0;
+    cudaError_t e = cudaStreamGetId(s, &id);
+    if (e != cudaSuccess || c->s_stream == 0 || id == c->s_stream) return e;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if ((e = cudaStreamIsCapturing(s, &st)) || st != cudaStreamCaptureStatusNone) return e;
+    if (!c->s_done && (e = cudaEventCreateWithFlags(&c->s_done, cudaEventDisableTiming))) return e;
+    if (c->s_on_own && (e = cudaEventRecord(c->s_done, c->stream))) return e;
+    return cudaStreamWaitEvent(s, c->s_done, 0);
+}
+// Behind the launch. (Nothing is recorded on the context's own stream until
+// another one follows: it lives as long as the context.)
+cudaError_t stateless_end(Ctx* c, cudaStream_t s) {
+    cudaError_t e;
+    if (s != c->stream) {
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        if ((e = cudaStreamIsCapturing(s, &st)) || st != cudaStreamCaptureStatusNone) return e;
+        if (!c->s_done && (e = cudaEventCreateWithFlags(&c->s_done, cudaEventDisableTiming))) return e;
+        if ((e = cudaEventRecord(c->s_done, s))) return e;
+    }
+    c->s_on_own = s == c->stream;
+    return cudaStreamGetId(s, &c->s_stream);
+}
+
 // Stage one block into the stateless scratch: descriptor + tile list (+ the
 // tensor map of its buffer for the TMA variant). *used = the variant the
 // tiles were built for (TMA falls back to GLOBAL for a buffer it cannot map).
@@ -648,6 +681,7 @@ int stage_single(Ctx* c, const granite_block_desc* b, double* u_dev, int* ntiles
                  int* used = nullptr) {
     int r = ensure_scratch(c, (size_t)cells_of(*b), 1);
     if (r) return r;
+    CK(stateless_begin(c, s), "order of the streams");
     DevBlock d = make_devblock(*b, c->p.ko_sigma);
     d.buf[0] = u_dev ? u_dev : c->s_u;
     if (variant == VARIANT_TMA) {
@@ -946,6 +980,7 @@ int granite_ccz4_destroy(void* h) {
     }
     for (auto e : c->pin_ev)
         if (e) cudaEventDestroy(e);
+    if (c->s_done) cudaEventDestroy(c->s_done);
     cudaFree(c->d_matter);
     cudaFree(c->s_diag);
     cudaFree(c->s_desc);
@@ -1074,6 +1109,7 @@ int granite_ccz4_compute_rhs_device(void* h, const granite_block_desc* b, const 
     a.coef_uniform = 1;
     a.coef = make_devblock(*b, c->p.ko_sigma);
     CK(launch_stage(variant, STORE_TILESET, precision, EPI_STORE, c->s_desc, c->s_tiles, nt, a, s), "launch RHS");
+    CK(stateless_end(c, s), "order of the streams");
     c->launches += 1;
     return GRANITE_OK;
 }
@@ -1176,6 +1212,7 @@ int granite_ccz4_apply_dissipation_host(void* h, const granite_block_desc* b, co
     CK(cudaMemcpyAsync(c->s_u, u, N * NV * sizeof(double), cudaMemcpyHostToDevice, s), "H2D u");
     CK(cudaMemcpyAsync(c->s_rhs, rhs, N * NV * sizeof(double), cudaMemcpyHostToDevice, s), "H2D rhs");
     CK(launch_dissipation(c->s_desc, 0, c->s_rhs, nt, c->s_tiles, s), "launch KO");
+    CK(stateless_end(c, s), "order of the streams");
     c->launches += 1;
     CK(cudaMemcpyAsync(rhs, c->s_rhs, N * NV * sizeof(double), cudaMemcpyDeviceToHost, s), "D2H rhs");
     CK(cudaStreamSynchronize(s), "sync");
@@ -1198,6 +1235,7 @@ int granite_ccz4_compute_constraints_host(void* h, const granite_block_desc* b, 
     // ham in s_rhs[0:N], mom in s_rhs[N:4N]; ghosts zero (ccz4.cpp:945-946)
     CK(cudaMemsetAsync(c->s_rhs, 0, 4 * N * sizeof(double), s), "memset");
     CK(launch_constraints(c->s_desc, c->s_tiles, nt, 0, c->s_rhs, c->s_rhs + N, nullptr, s), "launch constraints");
+    CK(stateless_end(c, s), "order of the streams");
     c->launches += 1;
     CK(cudaMemcpyAsync(ham, c->s_rhs, N * sizeof(double), cudaMemcpyDeviceToHost, s), "D2H ham");
     CK(cudaMemcpyAsync(mom, c->s_rhs + N, 3 * N * sizeof(double), cudaMemcpyDeviceToHost, s), "D2H mom");

@@ -133,7 +133,9 @@ GRANITE_API int granite_ccz4_compute_constraints_host(void* ctx, const granite_b
                                           const double* u, double* ham, double* mom);
 
 /* Same RHS on caller-owned device memory, enqueued on `stream` (a
- * cudaStream_t, NULL = the context stream). No host synchronisation. */
+ * cudaStream_t, NULL = the context stream). No host synchronisation. Calls of one
+ * context on different streams run one after the other on the device (they share
+ * the context's descriptor and tile list); contexts are independent. */
 GRANITE_API int granite_ccz4_compute_rhs_device(void* ctx, const granite_block_desc* b, const double* u_dev,
                                     double* rhs_dev, const double* rho_dev, const double* Si_dev,
                                     const double* Sij_dev, const double* S_dev, int precision,
