@@ -11,7 +11,6 @@
 
 #include <algorithm>
 #include <array>
-#include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
@@ -19,14 +18,13 @@
 #include <cstring>
 #include <map>
 #include <mutex>
-#include <system_error>
-#include <thread>
 #include <string>
 #include <tuple>
 #include <vector>
 
 #include "../../include/granite_ccz4.h"
 #include "ccz4_common.cuh"
+#include "ccz4_host_copy.h"
 #include "ccz4_kernels.h"
 
 using namespace granite_b200;
@@ -191,31 +189,6 @@ long long cells_of(const granite_block_desc& b) {
 
 }  // namespace
 
-// Copies between a caller's (pageable) buffers and the device: PIN_THREADS host
-// threads move pieces of up to PIN_SLOT bytes through pinned slots.
-constexpr int PIN_THREADS = 4;
-constexpr size_t PIN_SLOT = 512 << 10;
-// The pinned slots are shared by the contexts of the process (pinning memory
-// takes milliseconds, as long as the copies of a small block): one set, handed
-// to one call at a time and freed with the last context. A call that finds it
-// in use pins a set of its own context's.
-struct PinnedSet {
-    std::mutex in_use;  // held by the call that copies through it
-    std::mutex life;    // contexts and mem
-    int contexts = 0;
-    char* mem = nullptr;
-};
-PinnedSet g_pinned;
-
-char* alloc_pinned() {
-    void* p = nullptr;
-    if (cudaHostAlloc(&p, 2 * PIN_THREADS * PIN_SLOT, cudaHostAllocPortable) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    return static_cast<char*>(p);
-}
-
 struct Ctx {
     granite_ccz4_params p{};
     int device = 0;
@@ -272,12 +245,7 @@ struct Ctx {
     bool s_on_own = false;
     cudaEvent_t s_done = nullptr;
 
-    // pinned staging slots of the host-buffer copy at hand, two per copy thread,
-    // each with the event of its last copy; pin_own: this context's own set
-    char* s_pin = nullptr;
-    char* pin_own = nullptr;
-    bool counted = false;  // among g_pinned.contexts
-    cudaEvent_t pin_ev[2 * PIN_THREADS] = {};
+    HostCopy host_copy;  // staging of the host-buffer operator
 
     // resident hierarchy
     std::vector<granite_block_desc> descs;
@@ -505,145 +473,6 @@ int ensure_scratch(Ctx* c, size_t cells, int ntiles) {
         c->s_partials_cap = ntiles;
     }
     return GRANITE_OK;
-}
-
-// The staging slots of one call: the process's set, or the context's own.
-class PinnedLease {
-  public:
-    int take(Ctx* c) {
-        c_ = c;
-        for (auto& e : c->pin_ev)
-            if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate(staging)");
-        lock_ = std::unique_lock<std::mutex>(g_pinned.in_use, std::try_to_lock);
-        if (lock_.owns_lock()) {
-            std::lock_guard<std::mutex> life(g_pinned.life);
-            if (!g_pinned.mem) g_pinned.mem = alloc_pinned();
-            c->s_pin = g_pinned.mem;
-        } else {
-            if (!c->pin_own) c->pin_own = alloc_pinned();
-            c->s_pin = c->pin_own;
-        }
-        return c->s_pin ? GRANITE_OK : fail(c, GRANITE_ERR_NOMEM, "cudaHostAlloc(staging)");
-    }
-    // (every copy through the slots has been waited for, also after an error)
-    ~PinnedLease() {
-        if (!c_) return;
-        for (auto e : c_->pin_ev)
-            if (e) cudaEventSynchronize(e);
-        c_->s_pin = nullptr;
-    }
-
-  private:
-    Ctx* c_ = nullptr;
-    std::unique_lock<std::mutex> lock_;
-};
-
-// Run work(t, nt) on up to PIN_THREADS host threads (the caller's among them),
-// as many as `pieces` are worth; the first CUDA error of any of them.
-template <typename F>
-cudaError_t on_copy_threads(Ctx* c, size_t pieces, F&& work) {
-    const int hw = (int)std::thread::hardware_concurrency();
-    const int nt = (int)std::min<size_t>(std::max<size_t>(1, pieces / 2), (size_t)std::min(PIN_THREADS, hw > 0 ? hw : 1));
-    std::atomic<int> err{(int)cudaSuccess};
-    auto run = [&](int t, int n) {
-        cudaError_t e = cudaSetDevice(c->device);
-        if (e == cudaSuccess) e = work(t, n);
-        int none = (int)cudaSuccess;
-        if (e != cudaSuccess) err.compare_exchange_strong(none, (int)e);
-    };
-    std::thread th[PIN_THREADS];
-    int started = 1;
-    try {
-        for (; started < nt; ++started) th[started] = std::thread(run, started, nt);
-    } catch (const std::system_error&) {
-        // no more threads: the caller takes the rest of the shares
-    }
-    run(0, nt);
-    for (int t = started; t < nt; ++t) run(t, nt);
-    for (int t = 1; t < started; ++t) th[t].join();
-    return (cudaError_t)err.load();
-}
-
-// Host buffer -> device, queued on s when it returns (the host buffer is free
-// again). A copy straight from pageable memory is staged by one thread (12 GB/s).
-cudaError_t copy_in(Ctx* c, void* dst, const void* src, size_t bytes, cudaStream_t s) {
-    const size_t pieces = (bytes + PIN_SLOT - 1) / PIN_SLOT;
-    return on_copy_threads(c, pieces, [&](int t, int nt) {
-        for (size_t q = t, n = 0; q < pieces; q += nt, ++n) {
-            const int slot = 2 * t + (int)(n & 1);
-            const size_t off = q * PIN_SLOT, len = std::min(PIN_SLOT, bytes - off);
-            cudaError_t e = n >= 2 ? cudaEventSynchronize(c->pin_ev[slot]) : cudaSuccess;
-            if (e != cudaSuccess) return e;
-            std::memcpy(c->s_pin + slot * PIN_SLOT, static_cast<const char*>(src) + off, len);
-            e = cudaMemcpyAsync(static_cast<char*>(dst) + off, c->s_pin + slot * PIN_SLOT, len, cudaMemcpyHostToDevice, s);
-            if (e == cudaSuccess) e = cudaEventRecord(c->pin_ev[slot], s);
-            if (e != cudaSuccess) return e;
-        }
-        // the slots are reused by the next copy
-        for (int k = 0; k < 2; ++k) {
-            const cudaError_t e = cudaEventSynchronize(c->pin_ev[2 * t + k]);
-            if (e != cudaSuccess) return e;
-        }
-        return cudaSuccess;
-    });
-}
-
-// The interior cells of nv fields of block b, device -> host (both in the block's
-// layout; the host's ghost cells keep their values). Pieces are runs of rows of
-// one plane or of whole planes.
-cudaError_t copy_out_interior(Ctx* c, double* dst, const double* src, const granite_block_desc& b, int nv, cudaStream_t s) {
-    const size_t nx = b.ncells[0], ny = b.ncells[1], nz = b.ncells[2];
-    const size_t tx = nx + 2 * NG, ty = ny + 2 * NG, N = (size_t)cells_of(b);
-    const size_t row = tx * sizeof(double);
-    if (row > PIN_SLOT) {  // no row fits a slot
-        for (int v = 0; v < nv; ++v)
-            for (size_t k = 0; k < nz; ++k) {
-                const size_t at = v * N + ((k + NG) * ty + NG) * tx + NG;
-                const cudaError_t e = cudaMemcpy2DAsync(dst + at, row, src + at, row, nx * sizeof(double), ny,
-                                                        cudaMemcpyDeviceToHost, s);
-                if (e != cudaSuccess) return e;
-            }
-        return cudaStreamSynchronize(s);
-    }
-    const size_t rows_per = PIN_SLOT / row;
-    const size_t rows = ty * nz;                                 // of a field, from its first interior plane on
-    const size_t per_field = (rows + rows_per - 1) / rows_per, pieces = per_field * nv;
-    return on_copy_threads(c, pieces, [&](int t, int nt) {
-        size_t first[2] = {}, count[2] = {};  // the piece in each slot
-        double* base[2] = {};
-        auto finish = [&](int k) {
-            cudaError_t e = cudaEventSynchronize(c->pin_ev[2 * t + k]);
-            if (e != cudaSuccess) return e;
-            for (size_t q = 0; q < count[k]; ++q) {
-                const size_t j = (first[k] + q) % ty;
-                if (j < NG || j >= NG + ny) continue;
-                std::memcpy(base[k] + (first[k] + q) * tx + NG,
-                            reinterpret_cast<const double*>(c->s_pin + (2 * t + k) * PIN_SLOT) + q * tx + NG,
-                            nx * sizeof(double));
-            }
-            return cudaSuccess;
-        };
-        size_t n = 0;
-        for (size_t p = t; p < pieces; p += nt, ++n) {
-            const int k = (int)(n & 1);
-            cudaError_t e = n >= 2 ? finish(k) : cudaSuccess;
-            if (e != cudaSuccess) return e;
-            const size_t v = p / per_field;
-            first[k] = (p % per_field) * rows_per;
-            count[k] = std::min(rows_per, rows - first[k]);
-            const size_t origin = v * N + (size_t)NG * tx * ty;
-            base[k] = dst + origin;
-            e = cudaMemcpyAsync(c->s_pin + (2 * t + k) * PIN_SLOT, src + origin + first[k] * tx, count[k] * row,
-                                cudaMemcpyDeviceToHost, s);
-            if (e == cudaSuccess) e = cudaEventRecord(c->pin_ev[2 * t + k], s);
-            if (e != cudaSuccess) return e;
-        }
-        for (size_t m = n > 2 ? n - 2 : 0; m < n; ++m) {
-            const cudaError_t e = finish((int)(m & 1));
-            if (e != cudaSuccess) return e;
-        }
-        return cudaSuccess;
-    });
 }
 
 // A call on another stream than the last one's lets the last launch finish before
@@ -923,11 +752,7 @@ int granite_ccz4_create(const granite_ccz4_params* p, void** out) {
     if (cudaGetDeviceProperties(&prop, p->device) != cudaSuccess) return GRANITE_ERR_NO_DEVICE;
     if (prop.major != 10) return GRANITE_ERR_NO_DEVICE;  // kernels are built for sm_100a only
     Ctx* c = new Ctx();
-    {
-        std::lock_guard<std::mutex> life(g_pinned.life);
-        ++g_pinned.contexts;
-        c->counted = true;
-    }
+    c->host_copy.create(p->device);
     for (auto& row : c->class_cfg)
         for (int& k : row) k = AUTO_CFG;
     c->p = *p;
@@ -970,16 +795,7 @@ int granite_ccz4_destroy(void* h) {
     cudaFree(c->s_u);
     cudaFree(c->s_rhs);
     cudaFree(c->s_mat);
-    cudaFreeHost(c->pin_own);
-    {
-        std::lock_guard<std::mutex> life(g_pinned.life);
-        if (c->counted && --g_pinned.contexts == 0) {
-            cudaFreeHost(g_pinned.mem);
-            g_pinned.mem = nullptr;
-        }
-    }
-    for (auto e : c->pin_ev)
-        if (e) cudaEventDestroy(e);
+    c->host_copy.destroy();
     if (c->s_done) cudaEventDestroy(c->s_done);
     cudaFree(c->d_matter);
     cudaFree(c->s_diag);
@@ -1175,16 +991,15 @@ int granite_ccz4_compute_rhs_host(void* h, const granite_block_desc* b, const do
     cudaStream_t s = c->stream;
     // The kernel writes the interior cells and only they go back, so the caller's
     // rhs (whose ghost cells keep their values) need not be uploaded.
-    PinnedLease pinned;
-    if ((r = pinned.take(c))) return r;
-    CK(copy_in(c, c->s_u, u, N * NV * sizeof(double), s), "H2D u");
+    PinnedLease pinned(c->host_copy);
+    CK(copy_in(c->host_copy, c->s_u, u, N * NV * sizeof(double), s), "H2D u");
     const double *drho = nullptr, *dSi = nullptr, *dSij = nullptr, *dS = nullptr;
     if (nm == 4) {
         double* m = c->s_mat;
-        CK(copy_in(c, m, rho, N * sizeof(double), s), "H2D rho");
-        CK(copy_in(c, m + N, Si, 3 * N * sizeof(double), s), "H2D Si");
-        CK(copy_in(c, m + 4 * N, Sij, 6 * N * sizeof(double), s), "H2D Sij");
-        CK(copy_in(c, m + 10 * N, S, N * sizeof(double), s), "H2D S");
+        CK(copy_in(c->host_copy, m, rho, N * sizeof(double), s), "H2D rho");
+        CK(copy_in(c->host_copy, m + N, Si, 3 * N * sizeof(double), s), "H2D Si");
+        CK(copy_in(c->host_copy, m + 4 * N, Sij, 6 * N * sizeof(double), s), "H2D Sij");
+        CK(copy_in(c->host_copy, m + 10 * N, S, N * sizeof(double), s), "H2D S");
         drho = m;
         dSi = m + N;
         dSij = m + 4 * N;
@@ -1192,7 +1007,7 @@ int granite_ccz4_compute_rhs_host(void* h, const granite_block_desc* b, const do
     }
     r = granite_ccz4_compute_rhs_device(c, b, c->s_u, c->s_rhs, drho, dSi, dSij, dS, precision, s);
     if (r) return r;
-    CK(copy_out_interior(c, rhs, c->s_rhs, *b, NV, s), "D2H rhs");
+    CK(copy_out_interior(c->host_copy, rhs, c->s_rhs, b->ncells, NV, s), "D2H rhs");
     CK(cudaStreamSynchronize(s), "sync");
     return check_errflag(c);
 }

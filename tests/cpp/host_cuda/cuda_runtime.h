@@ -14,3 +14,23 @@ struct int2 {
 };
 inline double __dadd_rn(double a, double b) { return a + b; }
 inline double __dmul_rn(double a, double b) { return a * b; }
+
+// The runtime calls of the host code under test; each test defines its own.
+#include <cstddef>
+
+enum cudaError_t { cudaSuccess = 0, cudaErrorInvalidValue = 1, cudaErrorMemoryAllocation = 2 };
+enum cudaMemcpyKind { cudaMemcpyHostToDevice = 1, cudaMemcpyDeviceToHost = 2 };
+enum { cudaHostAllocPortable = 1, cudaEventDisableTiming = 2 };
+using cudaStream_t = struct FakeStream*;
+using cudaEvent_t = struct FakeEvent*;
+cudaError_t cudaHostAlloc(void**, size_t, unsigned);
+cudaError_t cudaFreeHost(void*);
+cudaError_t cudaGetLastError();
+cudaError_t cudaSetDevice(int);
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t*, unsigned);
+cudaError_t cudaEventDestroy(cudaEvent_t);
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t);
+cudaError_t cudaEventSynchronize(cudaEvent_t);
+cudaError_t cudaMemcpyAsync(void*, const void*, size_t, cudaMemcpyKind, cudaStream_t);
+cudaError_t cudaMemcpy2DAsync(void*, size_t, const void*, size_t, size_t, size_t, cudaMemcpyKind, cudaStream_t);
+cudaError_t cudaStreamSynchronize(cudaStream_t);

@@ -1,6 +1,7 @@
-"""Host parts of the stage kernel without a device: its ring protocol on host threads
-(tests/cpp/test_stage_ring.cpp: load warp and compute warps with waits that run
-out in some lanes only) and the table of kernels that may be launched."""
+"""Parts of the library that a host compiler can run without a device
+(tests/cpp): the stage kernel's ring protocol on host threads, with waits that run
+out in some lanes only; the table of kernels that may be launched; the staged
+copies of the host-buffer operator over a fake runtime."""
 import os
 import subprocess
 
@@ -35,4 +36,10 @@ def test_ring(exe, what):
 
 def test_every_kernel_answers_for_its_registers(tmp_path):
     r = subprocess.run([build(tmp_path, "test_tma_grids")], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("what", ["staged", "no_pinned", "no_events", "copy_error"])
+def test_host_copies(tmp_path, what):
+    r = subprocess.run([build(tmp_path, "test_host_copy"), what], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout + r.stderr
