@@ -6,8 +6,8 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <exception>
 #include <mutex>
-#include <system_error>
 #include <thread>
 
 #include "ccz4_common.cuh"
@@ -119,8 +119,9 @@ cudaError_t on_copy_threads(const HostCopy& c, size_t pieces, F&& work) {
     int started = 1;
     try {
         for (; started < nt; ++started) th[started] = std::thread(run, started, nt);
-    } catch (const std::system_error&) {
-        // no more threads: the caller takes the rest of the shares
+    } catch (const std::exception&) {
+        // no thread left (system_error) or no memory for one (bad_alloc): the caller
+        // takes the rest of the shares
     }
     run(0, nt);
     for (int t = started; t < nt; ++t) run(t, nt);

@@ -1,14 +1,34 @@
 // The staged copies of the host-buffer operator (ccz4_host_copy.h) over a fake
 // runtime whose "device" is host memory: with slots, where no memory can be
-// pinned and where no event can be made, for blocks of one piece, of many with a
+// pinned, where no event can be made, and where a thread cannot be started (none
+// left, or no memory for its state), for blocks of one piece, of many with a
 // ragged last one, and of rows wider than a slot.
+#include <dlfcn.h>
+#include <pthread.h>
+
+#include <cerrno>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <new>
 #include <string>
 #include <vector>
 
 #include "ccz4_host_copy.h"
+
+static bool copying = false;                            // within a copy:
+static bool no_threads = false, no_thread_state = false;  // what fails there
+
+extern "C" int pthread_create(pthread_t* t, const pthread_attr_t* a, void* (*f)(void*), void* x) noexcept {
+    static const auto real = reinterpret_cast<decltype(&pthread_create)>(dlsym(RTLD_NEXT, "pthread_create"));
+    return copying && no_threads ? EAGAIN : real(t, a, f, x);
+}
+void* operator new(size_t n) {
+    if (void* p = copying && no_thread_state ? nullptr : std::malloc(n ? n : 1)) return p;
+    throw std::bad_alloc();
+}
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, size_t) noexcept { std::free(p); }
 
 static bool no_pinned = false, no_events = false, no_copies = false;
 static int pinned = 0, events = 0;
@@ -62,8 +82,10 @@ static int round_trip(const int n[3], int nv) {
     int bad = 0;
     for (int again = 0; again < 2; ++again) {
         PinnedLease lease(c);
+        copying = true;
         bad += copy_in(c, dev.data(), u.data(), u.size() * sizeof(double), nullptr) != cudaSuccess;
         bad += copy_out_interior(c, back.data(), dev.data(), n, nv, nullptr) != cudaSuccess;
+        copying = false;
     }
     bad += dev != u;
     auto inner = [&](size_t i, int d) { return i >= (size_t)NG && i < (size_t)(NG + n[d]); };
@@ -80,6 +102,8 @@ int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     no_pinned = what == "no_pinned";
     no_events = what == "no_events";
+    no_threads = what == "no_threads";
+    no_thread_state = what == "no_thread_state";
     const int small[3] = {5, 3, 2}, many[3] = {64, 40, 33}, wide[3] = {65600, 2, 1};
     int bad = round_trip(small, 22) + round_trip(many, 22) + round_trip(wide, 2);
     if (what == "copy_error") {  // an error of a copy is the call's

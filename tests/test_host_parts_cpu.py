@@ -13,7 +13,7 @@ CXX = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
 
 def build(out, name):
     cpp = os.path.join(ROOT, "tests", "cpp")
-    subprocess.run([CXX, "-std=c++17", "-O1", "-pthread", "-I", os.path.join(cpp, "host_cuda"),
+    subprocess.run([CXX, "-std=c++17", "-O1", "-pthread", "-ldl", "-I", os.path.join(cpp, "host_cuda"),
                     "-I", os.path.join(ROOT, "granite_b200", "csrc"), os.path.join(cpp, name + ".cpp"),
                     "-o", str(out / name)], check=True)
     return str(out / name)
@@ -39,7 +39,7 @@ def test_every_kernel_answers_for_its_registers(tmp_path):
     assert r.returncode == 0, r.stdout + r.stderr
 
 
-@pytest.mark.parametrize("what", ["staged", "no_pinned", "no_events", "copy_error"])
+@pytest.mark.parametrize("what", ["staged", "no_pinned", "no_events", "no_threads", "no_thread_state", "copy_error"])
 def test_host_copies(tmp_path, what):
     r = subprocess.run([build(tmp_path, "test_host_copy"), what], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout + r.stderr
