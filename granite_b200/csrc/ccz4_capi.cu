@@ -1502,13 +1502,12 @@ int granite_ccz4_download_block(void* h, int i, double* host) {
 // then the FP32 kernel over the unflagged tiles and the FP64 kernel over the
 // flagged ones. The two passes write disjoint tiles, so the in-place last
 // stage is safe and no tile is computed twice.
-// block >= 0: the tiles are that block's alone, else the blocks of the level.
 static cudaError_t stage_range(Ctx* c, LevelLists& L, int tileset, int precision, const StageArgs& a0, int first,
-                               int count, long long* n, int block = -1) {
+                               int count, long long* n) {
     const Tile* tiles = L.d_tiles + first;
     StageArgs a = a0;
-    a.coef_uniform = block >= 0 || L.uniform;
-    a.coef = c->hblocks[block >= 0 ? block : L.blocks[0]];
+    a.coef_uniform = L.uniform;  // the level's, also block by block: the same kernel and bits
+    a.coef = c->hblocks[L.blocks[0]];
     if (L.variant == VARIANT_TMA) {  // the tensor maps of the box shapes
         const size_t shape = 3 * c->descs.size();
         a.tmaps = c->d_tmaps;
@@ -1562,7 +1561,7 @@ static cudaError_t level_stage(Ctx* c, LevelLists& L, int precision, const Stage
     for (size_t q = 0; q < L.tile_range[pr].size(); ++q) {
         const auto& r = L.tile_range[pr][q];
         cudaError_t e = timed(c, GRANITE_KERNEL_STAGE, [&] {
-            return stage_range(c, L, L.block_tiles[pr][q], precision, a, r.first, r.second, n, L.blocks[q]);
+            return stage_range(c, L, L.block_tiles[pr][q], precision, a, r.first, r.second, n);
         });
         if (e != cudaSuccess) return e;
     }

@@ -385,7 +385,11 @@ GRANITE_API int granite_ccz4_profile_get(void* ctx, int kernel_class, double* to
  * send their level to GRANITE_VARIANT_GLOBAL. A TMA load that does not complete
  * within its wait limit makes the next granite_ccz4_sync, block download
  * (download_block / download_all) or compute_rhs_host return GRANITE_ERR_CUDA.
- * All variants compute identical FP64 results. */
+ * All variants compute identical FP64 results. In GRANITE_VARIANT_TMA a level
+ * whose blocks all have one spacing (to the last bit) runs a form of the kernel
+ * that takes the stencil coefficients as arguments, any other level one that reads
+ * each block's: FP64 results are the same bits in both, mixed results may
+ * differ in the rounding of the FP32 algebra (1e-8 of a field's scale after two steps). */
 #define GRANITE_VARIANT_GLOBAL 0
 #define GRANITE_VARIANT_SMEM 1
 #define GRANITE_VARIANT_GLOBAL_R168 2 /* GLOBAL with at most 168 registers (3 CTAs / SM) */
@@ -471,7 +475,8 @@ GRANITE_API int granite_ccz4_set_ghost_push(void* ctx, int on);
 /* Batching (no counterpart in the reference): 1 (default) = one launch per
  * level and RK stage over all blocks, each step replayed as one CUDA graph;
  * 0 = one launch per block and stage, issued eagerly, as a per-block drop-in
- * of the reference's per-GridBlock operator calls would run. */
+ * of the reference's per-GridBlock operator calls would run. The results are
+ * the same bits. */
 GRANITE_API int granite_ccz4_set_batching(void* ctx, int batched);
 
 /* The context's cudaStream_t, for callers that order their own work or events

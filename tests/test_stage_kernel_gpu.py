@@ -61,10 +61,12 @@ def test_fp64_steps_match_the_oracle(gb, oracle_lib, n, cfg):
 
 @pytest.mark.parametrize("precision,chi", [(0, 0.0), (1, 0.0), (1, 0.5), (1, 0.999999)])
 def test_blocks_of_different_spacing_share_a_launch(gb, oracle_lib, precision, chi):
-    """Blocks whose coefficients differ are read from their descriptors in a
-    batched launch and from the kernel arguments block by block. The two kernels
-    may contract the algebra differently: a few units in the last place of the
-    RHS per stage in FP64 (6 stages, below 1e-13), of FP32 in the mixed form."""
+    """The kernel reads the coefficients of a level whose blocks differ in them from
+    the descriptors, one launch for the level or one per block: the same kernel,
+    the same bits. A block alone has its coefficients in the kernel arguments. The
+    two kernels may contract the algebra differently: a few units in the last
+    place of the RHS per stage in FP64 (6 stages, below 1e-13), of FP32 in the
+    mixed form."""
     geoms = [Geom((24, 20, 16), (-3.0, -2.5, -2.0), (3.0, 2.5, 2.0)),
              Geom((32, 16, 18), (4.0, 4.0, 4.0), (13.6, 9.2, 9.7)),
              Geom((18, 22, 14), (-9.0, -9.0, -9.0), (-4.5, -3.5, -5.5))]
@@ -72,7 +74,10 @@ def test_blocks_of_different_spacing_share_a_launch(gb, oracle_lib, precision, c
     a, _ = _run(gb, geoms, states, precision, True, chi)
     b, _ = _run(gb, geoms, states, precision, False, chi)
     for i in range(len(geoms)):
-        parity(a[i], b[i], rtol=1e-13 if precision == 0 else 1e-6, what=f"block {i}")
+        assert np.array_equal(a[i], b[i]), f"block {i}: batched and block by block"
+    # (the first block: the step length is its own)
+    (alone,), _ = _run(gb, geoms[:1], states[:1], precision, True, chi)
+    parity(a[0], alone, rtol=1e-13 if precision == 0 else 1e-6, what="the first block alone")
 
 
 # 24^3 cells of 8 bytes are less than a staging piece; 64 x 40: a field is several
