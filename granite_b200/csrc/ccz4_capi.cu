@@ -26,6 +26,7 @@
 #include "ccz4_common.cuh"
 #include "ccz4_host_copy.h"
 #include "ccz4_kernels.h"
+#include "ccz4_restrict_list.h"
 
 using namespace granite_b200;
 
@@ -1731,31 +1732,9 @@ int level_grid(Ctx* c, std::vector<std::array<int, 3>>& G) {
     return GRANITE_OK;
 }
 
-// The restriction boxes into a level (x.dst coarse, x.src fine, children of the
-// box's first cell at x.s0) as one list with each coarse cell once: where boxes
-// overlap the last one decides, as when they run one after the other (a box
-// reads only cells of the finer level).
 int upload_restriction(Ctx* c, const std::vector<XferBox>& boxes, LevelXfer& X) {
-    std::map<int, std::vector<GhostSrc>> cells;  // per coarse block
-    for (const XferBox& x : boxes) {
-        const auto& d = c->descs[x.dst];
-        const auto& f = c->descs[x.src];
-        const int T0 = d.ncells[0] + 2 * NG, T1 = d.ncells[1] + 2 * NG, T2 = d.ncells[2] + 2 * NG;
-        const int S0 = f.ncells[0] + 2 * NG, S1 = f.ncells[1] + 2 * NG;
-        auto& m = cells[x.dst];
-        if (m.empty()) m.assign((size_t)T0 * T1 * T2, GhostSrc{-1, 0, 0, 0});
-        for (int k = 0; k < x.n[2]; ++k)
-            for (int j = 0; j < x.n[1]; ++j)
-                for (int i = 0; i < x.n[0]; ++i) {
-                    const int cell = x.d0[0] + i + T0 * (x.d0[1] + j + T1 * (x.d0[2] + k));
-                    m[cell] = GhostSrc{x.dst, cell, x.src,
-                                       x.s0[0] + 2 * i + S0 * (x.s0[1] + 2 * j + S1 * (x.s0[2] + 2 * k))};
-                }
-    }
-    std::vector<GhostSrc> items;
-    for (const auto& kv : cells)
-        for (const GhostSrc& g : kv.second)
-            if (g.dst_block >= 0) items.push_back(g);
+    const std::vector<GhostSrc> items =
+        restriction_list(boxes, [&](int b, int d) { return c->descs[b].ncells[d] + 2 * NG; });
     CK(upload_vec(items, &X.d_restrict, c->stream), "upload restriction list");
     X.nrestrict = (long long)items.size();
     return GRANITE_OK;

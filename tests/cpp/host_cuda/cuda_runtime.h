@@ -12,6 +12,9 @@
 struct int2 {
     int x, y;
 };
+struct double2 {
+    double x, y;
+};
 inline double __dadd_rn(double a, double b) { return a + b; }
 inline double __dmul_rn(double a, double b) { return a * b; }
 

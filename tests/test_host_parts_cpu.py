@@ -1,7 +1,7 @@
 """Parts of the library that a host compiler can run without a device
 (tests/cpp): the stage kernel's ring protocol on host threads, with waits that run
 out in some lanes only; the table of kernels that may be launched; the staged
-copies of the host-buffer operator over a fake runtime."""
+copies of the host-buffer operator over a fake runtime; the list of restricted cells."""
 import os
 import subprocess
 
@@ -42,4 +42,9 @@ def test_every_kernel_answers_for_its_registers(tmp_path):
 @pytest.mark.parametrize("what", ["staged", "no_pinned", "no_events", "no_threads", "no_thread_state", "copy_error"])
 def test_host_copies(tmp_path, what):
     r = subprocess.run([build(tmp_path, "test_host_copy"), what], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_restriction_list(tmp_path):
+    r = subprocess.run([build(tmp_path, "test_restrict_list")], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout + r.stderr
