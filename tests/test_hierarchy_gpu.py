@@ -160,21 +160,25 @@ def test_hierarchy_mixed_close_to_fp64(gb, oracle_lib):
         parity(b, a, rtol=1e-5, what="mixed vs fp64")
 
 
+@pytest.mark.parametrize("mode", ["ghosts", "reference"])
 @pytest.mark.parametrize("precision,layout", [(0, "small"), (1, "small"), (0, "tma"), (1, "tma")])
-def test_finest_prefill_skip_is_exact(gb, oracle_lib, precision, layout):
+def test_finest_prefill_skip_is_exact(gb, oracle_lib, precision, layout, mode):
     # the graph-captured step leaves out the fill before the finest level's second
     # substep (its inputs are those of the fill that ended the first one), and
     # once the fill after a level's step has made its same-level copies current,
     # its fill before the next step copies only cells whose source a restriction
     # rewrote in between (within a coarse step and across coarse steps); the
     # uncaptured step with the regrid hook (interval 0: no regrid) performs every
-    # fill in full, as amr.cpp does: the two agree bit for bit
+    # fill in full, as amr.cpp does: the two agree bit for bit (in the reference's
+    # mode that fill also prolongates the whole finest level)
+    amr = gb.AMR_GHOSTS if mode == "ghosts" else gb.AMR_REFERENCE
     if layout == "small":
         h, geoms, levels = small_hierarchy(seed=17, levels=3)
     else:  # blocks of 16 to 32 cells (the TMA stage kernel on every level)
         from granite_b200.hierarchy import make_binary_hierarchy
-        h = make_binary_hierarchy(seed=23, levels=3, coarse_n=48, extent=16.0, sizes=(16, 24, 32),
-                                  blocks_per_level=(8, 40))
+        # (the reference's restriction rounds cell positions: exact spacings there)
+        h = make_binary_hierarchy(seed=23, levels=3, coarse_n=48 if mode == "ghosts" else 64, extent=16.0,
+                                  sizes=(16, 24, 32), blocks_per_level=(8, 40))
         geoms = [Geom(b.ncells, b.lo, b.hi) for b in h.blocks]
         levels = [b.level for b in h.blocks]
     states = [oracle.add_noise(oracle_lib.init_brill_lindquist(g, h.masses, h.positions, r_floor=0.5 * g.dx[0]),
@@ -186,9 +190,9 @@ def test_finest_prefill_skip_is_exact(gb, oracle_lib, precision, layout):
         ev.set_fp64_chi_threshold(0.5)
         for _ in range(3):
             if hooked:
-                ev.hierarchy_step_regrid(dt, None, 0, precision=precision, amr_mode=gb.AMR_GHOSTS)
+                ev.hierarchy_step_regrid(dt, None, 0, precision=precision, amr_mode=amr)
             else:
-                ev.hierarchy_step(dt, precision, gb.AMR_GHOSTS)
+                ev.hierarchy_step(dt, precision, amr)
         ev.download()
         outs.append([b.array.copy() for b in blocks])
         ev.close()
