@@ -527,7 +527,7 @@ def main():
     ap.add_argument("--accuracy-seconds", type=float, default=420.0,
                     help="wall-time cap of the accuracy run")
     ap.add_argument("--stage-config", type=int, default=-1,
-                    help="one TMA stage-kernel configuration for every block (default: the per-class table)")
+                    help="one TMA stage-kernel configuration for every block (default: the library chooses tiles per level)")
     ap.add_argument("--ghost-push", type=int, default=-1, choices=[-1, 0, 1],
                     help="GRANITE_AMR_GHOSTS: stage kernels write the same-level ghost copies (1) or the "
                          "fills copy them (0); -1 = the library default")

@@ -35,6 +35,7 @@ VARIANT_GLOBAL, VARIANT_SMEM, VARIANT_GLOBAL_R168, VARIANT_GLOBAL_R128, VARIANT_
 VARIANT_NAMES = {"global": 0, "smem": 1, "global_r168": 2, "global_r128": 3, "tma": 4}
 # configurations of the TMA stage kernel and the block-size classes they are tuned for
 STAGE_CONFIGS = 18
+STAGE_TILE_SET_CONFIGS = (0, 12)  # an id per tile set: without and with x-remainder tiles
 STAGE_CLASS_EDGES = (16, 24, 32, 48, 64, 96)
 
 _ERRORS = {-1: "invalid argument", -2: "CUDA error", -3: "no sm_100 device", -4: "out of memory",
@@ -179,7 +180,7 @@ def _dp(a):
 # ---------------------------------------------------------------------------
 
 def stage_config_info(cfg: int) -> dict:
-    """Tile depth, ring slots, shared-memory options and schedule of a TMA configuration."""
+    """The kernel and tile set a TMA configuration id runs (include/granite_ccz4.h)."""
     lib = load_library()
     v = [C.c_int() for _ in range(4)]
     rc = lib.granite_ccz4_stage_config_info(int(cfg), *[C.byref(x) for x in v])
@@ -483,7 +484,7 @@ class Evolver:
         self.ctx.check(self.ctx.lib.granite_ccz4_set_ghost_push(self.ctx.h, int(bool(on))))
 
     def set_pass_overlap(self, on: bool):
-        """Per-tile precision: the FP64 pass beside the FP32 pass on a second stream (default) or after it."""
+        """Per-tile precision: the FP64 pass beside the FP32 pass on a second stream, or after it (default)."""
         self.ctx.check(self.ctx.lib.granite_ccz4_set_pass_overlap(self.ctx.h, int(bool(on))))
 
     def set_batching(self, batched: bool):
@@ -495,12 +496,13 @@ class Evolver:
         self.ctx.check(self.ctx.lib.granite_ccz4_set_stage_config(self.ctx.h, int(precision), int(cls), int(cfg)))
 
     def stage_config(self, precision: int, cls: int) -> int:
+        """The configuration set for the class, or after commit an id of the tile set its blocks run."""
         v = C.c_int()
         self.ctx.check(self.ctx.lib.granite_ccz4_get_stage_config(self.ctx.h, int(precision), int(cls), C.byref(v)))
         return v.value
 
     def force_stage_config(self, cfg: int):
-        """One TMA configuration for every block and precision (-1: the per-class table). Before commit."""
+        """One TMA configuration for every block and precision (-1: each class's own). Before commit."""
         self.ctx.check(self.ctx.lib.granite_ccz4_force_stage_config(self.ctx.h, int(cfg)))
 
     def apply_stage_table(self, table: dict):

@@ -72,10 +72,10 @@ bool encode_block_tmap(void* map128, const double* base, const DevBlock& d, int 
 
 namespace {
 
-// The configuration granite_ccz4_get_stage_config reports for a class without
-// one of its own; which tile set a level then runs is level_default_tileset's
-// choice.
-constexpr int DEFAULT_CFG = 12;
+// The configuration granite_ccz4_get_stage_config reports per precision (FP64,
+// MIXED) for a class that was given none and that no committed block is of. Which
+// tile set a level runs is level_default_tileset's choice.
+constexpr int DEFAULT_CFG[2] = {0, 12};
 
 // A table entry or forced configuration that leaves the choice to the library.
 constexpr int AUTO_CFG = -1;
@@ -643,8 +643,14 @@ int granite_ccz4_get_stage_config(const void* h, int precision, int cls, int* cf
     const Ctx* c = static_cast<const Ctx*>(h);
     if (!c || !cfg || cls < 0 || cls >= GRANITE_STAGE_CLASSES) return GRANITE_ERR_INVALID;
     if (precision != GRANITE_PRECISION_FP64 && precision != GRANITE_PRECISION_MIXED) return GRANITE_ERR_INVALID;
-    *cfg = c->forced_cfg >= 0 ? c->forced_cfg : c->class_cfg[precision == GRANITE_PRECISION_MIXED ? 1 : 0][cls];
-    if (*cfg == AUTO_CFG) *cfg = DEFAULT_CFG;
+    const int pr = precision == GRANITE_PRECISION_MIXED ? 1 : 0;
+    *cfg = c->forced_cfg >= 0 ? c->forced_cfg : c->class_cfg[pr][cls];
+    if (*cfg != AUTO_CFG) return GRANITE_OK;
+    long long blocks[NUM_TMA_TILESETS] = {};  // of the class, by the tile set they run
+    for (const LevelLists& L : c->levels)
+        for (size_t q = 0; q < L.block_tiles[pr].size(); ++q)
+            if (L.variant == VARIANT_TMA && stage_class_of(c->descs[L.blocks[q]]) == cls) ++blocks[L.block_tiles[pr][q]];
+    *cfg = blocks[0] + blocks[1] == 0 ? DEFAULT_CFG[pr] : TMA_TILESET_CFG[blocks[1] > blocks[0] ? 1 : 0];
     return GRANITE_OK;
 }
 
@@ -659,20 +665,20 @@ int granite_ccz4_force_stage_config(void* h, int cfg) {
 
 int granite_ccz4_stage_config_info(int cfg, int* tile_z, int* ring_slots, int* shared_input, int* shared_hessian) {
     if (cfg < 0 || cfg >= NUM_TMA_CFGS) return GRANITE_ERR_INVALID;
-    if (tile_z) *tile_z = TMA_CFGS[cfg].tz;
-    if (ring_slots) *ring_slots = TMA_CFGS[cfg].nbuf;
-    if (shared_input) *shared_input = TMA_CFGS[cfg].tin;
-    if (shared_hessian) *shared_hessian = TMA_CFGS[cfg].hs;
+    if (tile_z) *tile_z = TMA_TZ;
+    if (ring_slots) *ring_slots = TMA_SLOTS_MIXED;
+    if (shared_input) *shared_input = 0;
+    if (shared_hessian) *shared_hessian = 0;
     return GRANITE_OK;
 }
 
 int granite_ccz4_stage_config_schedule(int cfg, int* warp_specialized, int* ctas_per_sm, int* items_per_barrier,
                                        int* x_remainder_tiles) {
     if (cfg < 0 || cfg >= NUM_TMA_CFGS) return GRANITE_ERR_INVALID;
-    if (warp_specialized) *warp_specialized = TMA_CFGS[cfg].ws;
-    if (ctas_per_sm) *ctas_per_sm = TMA_CFGS[cfg].minb;
-    if (items_per_barrier) *items_per_barrier = TMA_CFGS[cfg].bar;
-    if (x_remainder_tiles) *x_remainder_tiles = TMA_CFGS[cfg].rem;
+    if (warp_specialized) *warp_specialized = 1;
+    if (ctas_per_sm) *ctas_per_sm = 1;
+    if (items_per_barrier) *items_per_barrier = 1;
+    if (x_remainder_tiles) *x_remainder_tiles = tma_tileset(cfg);
     return GRANITE_OK;
 }
 static_assert(GRANITE_STAGE_CONFIGS == NUM_TMA_CFGS, "the header's configuration count");

@@ -24,34 +24,19 @@ enum {
 // Tile shape of a stage-kernel variant (points along x, y, z).
 void stage_tile_dims(int variant, int* tx, int* ty, int* tz);
 
-// The table of configuration ids of the TMA variant: what a caller may set per
-// precision and block-size class, and what granite_ccz4_stage_config_info tells
-// of each. They were the candidates of the kernel that issued its own loads (its
-// tile depth, ring slots, shared-memory options, CTAs per SM and barrier
-// grouping). The kernel with load warps (ccz4_stage_tma.cuh) is faster than the
-// best of them for every block size and precision (mixed 343 against 411 us,
-// FP64 470 against 501 on 128 x 128 x 64 points), so an id now chooses between
-// its two tile sets only (tma_tileset): x-remainder tiles or not.
-struct TmaCfg {
-    int tz, nbuf, tin, hs, ws, minb, bar;
-    // x-remainder tiles: a block whose x extent leaves 8 cells after its 16-wide
-    // tiles covers them with 8 x 4 x 4 tiles (Tile::w = -8, every thread on a
-    // point) instead of 16-wide tiles half outside the block
-    int rem;
-    int pf;
-};
-constexpr int NUM_TMA_CFGS = 18;
-constexpr TmaCfg TMA_CFGS[NUM_TMA_CFGS] = {
-    {4, 3, 0, 0, 0, 1, 1, 0, 0}, {4, 3, 1, 1, 0, 1, 1, 0, 0}, {2, 3, 1, 1, 0, 2, 1, 0, 0},
-    {2, 2, 1, 1, 0, 2, 1, 0, 0}, {2, 3, 1, 0, 0, 2, 1, 0, 0}, {2, 3, 0, 0, 1, 2, 1, 0, 0},
-    {2, 3, 0, 0, 0, 3, 1, 0, 0}, {2, 2, 1, 0, 0, 3, 1, 0, 0}, {2, 3, 1, 0, 0, 2, 2, 0, 0},
-    {2, 4, 0, 0, 0, 2, 2, 0, 0}, {4, 4, 0, 0, 0, 1, 2, 0, 0}, {2, 3, 1, 0, 0, 2, 1, 1, 0},
-    {2, 3, 0, 0, 0, 2, 1, 1, 0}, {2, 2, 1, 0, 0, 2, 1, 1, 0}, {2, 3, 0, 0, 0, 2, 1, 1, 1},
-    {4, 4, 0, 0, 0, 1, 2, 1, 0}, {4, 4, 0, 0, 0, 1, 2, 2, 0}, {2, 4, 0, 0, 0, 2, 2, 2, 0}};
 // Tile sets of the TMA kernel: 0 = 16 x 4 x 2 tiles (and the store epilogue of the
-// drop-in RHS), 1 = with x-remainder tiles.
+// drop-in RHS), 1 = with x-remainder tiles: a block whose x extent leaves 8 cells
+// after its 16-wide tiles covers them with 8 x 4 x 4 tiles (Tile::w = -8, every
+// thread on a point) instead of 16-wide tiles half outside the block.
 constexpr int NUM_TMA_TILESETS = 2;
-constexpr int tma_tileset(int cfg) { return TMA_CFGS[cfg].rem ? 1 : 0; }
+// A configuration id, what a caller may set per precision and block-size class,
+// stands for a tile set: those below TMA_FIRST_REM_CFG for set 0, the others for
+// set 1. TMA_TILESET_CFG: the id reported for a set that the library chose.
+constexpr int NUM_TMA_CFGS = 18, TMA_FIRST_REM_CFG = 11;
+constexpr int tma_tileset(int cfg) { return cfg < TMA_FIRST_REM_CFG ? 0 : 1; }
+constexpr int TMA_TILESET_CFG[NUM_TMA_TILESETS] = {0, 12};
+// Ring slots per compute warpgroup of the mixed and of the FP64 kernels.
+constexpr int TMA_SLOTS_MIXED = 3, TMA_SLOTS_FP64 = 4;
 constexpr int TMA_TZ = 2;
 // Points of an x-remainder tile along x.
 constexpr int TMA_REM_X = 8;

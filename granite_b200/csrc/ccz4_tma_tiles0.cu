@@ -6,7 +6,7 @@
 #include "ccz4_stage_tma.cuh"
 
 namespace granite_b200 {
-using Ops0 = TmaKernelOps<TmaKernelT<3, 3, false>, TmaKernelT<2, 4, false>>;
+using Ops0 = TmaKernelOps<TmaKernelT<3, TMA_SLOTS_MIXED, false>, TmaKernelT<2, TMA_SLOTS_FP64, false>>;
 cudaError_t configure_tma_tiles0(int nsm, TmaGrids& grids) { return Ops0::configure<true>(nsm, grids); }
 cudaError_t launch_tma_tiles0(int pm, int epi, bool sel, const DevBlock* blocks, const Tile* tiles, int ntiles,
                               const StageArgs& args, cudaStream_t stream, int grid) {

@@ -6,7 +6,7 @@
 #include "ccz4_stage_tma.cuh"
 
 namespace granite_b200 {
-using Ops1 = TmaKernelOps<TmaKernelT<3, 3, true>, TmaKernelT<2, 4, true>>;
+using Ops1 = TmaKernelOps<TmaKernelT<3, TMA_SLOTS_MIXED, true>, TmaKernelT<2, TMA_SLOTS_FP64, true>>;
 cudaError_t configure_tma_tiles1(int nsm, TmaGrids& grids) { return Ops1::configure<false>(nsm, grids); }
 cudaError_t launch_tma_tiles1(int pm, int epi, bool sel, const DevBlock* blocks, const Tile* tiles, int ntiles,
                               const StageArgs& args, cudaStream_t stream, int grid) {

@@ -3,17 +3,18 @@
 The reference evaluates computeRHS with one OpenMP loop per block whatever its
 size (ccz4.cpp:267-270). Here a configuration id chooses the stage kernel's
 tiles (granite_b200.stage_config_info: with x-remainder tiles or without), and
-the better choice depends on the block size and on the precision. For every block-size class (edge
-in STAGE_CLASS_EDGES) and precision this module times every configuration on a
-level of equal cubic blocks of that edge carrying single-puncture data (about
-two million interior points, so a launch takes about a millisecond), with CUDA
-events around every stage launch (the library's profiler), and keeps the
-fastest. The result is a table {"fp64": [cfg per class], "mixed": [...]} that
-Evolver.apply_stage_table applies, and a uniform table (one configuration per
-precision for every class). A level whose blocks use different tiles runs one
-launch per tile set; without a table the library chooses one set per level.
+the better choice depends on the block size and on the precision. For every
+block-size class (edge in STAGE_CLASS_EDGES) and precision this module times one
+configuration of each tile set on a level of equal cubic blocks of that edge
+carrying single-puncture data (about two million interior points, so a launch
+takes about a millisecond), with CUDA events around every stage launch (the
+library's profiler), and keeps the fastest. The result is a table
+{"fp64": [cfg per class], "mixed": [...]} that Evolver.apply_stage_table applies,
+and a uniform table (one configuration per precision for every class). A level
+whose blocks use different tiles runs one launch per tile set; without a table
+the library chooses one set per level.
 
-    python -m granite_b200.tuner [--out table.json] [--classes 16,24] [--configs 0,4] [--precisions mixed]
+    python -m granite_b200.tuner [--out table.json] [--classes 16,24] [--configs 0,12] [--precisions mixed]
                                  [--steps 3]
 """
 from __future__ import annotations
@@ -26,7 +27,7 @@ import time
 
 import numpy as np
 
-from . import (PRECISION_FP64, PRECISION_MIXED, STAGE_CLASS_EDGES, STAGE_CONFIGS, BC_REFERENCE, CCZ4Params,
+from . import (PRECISION_FP64, PRECISION_MIXED, STAGE_CLASS_EDGES, STAGE_TILE_SET_CONFIGS, BC_REFERENCE, CCZ4Params,
                Evolver, GridBlock, KERNEL_STAGE, block_stage_class, stage_config_info)
 from .initial_data import add_noise, brill_lindquist
 
@@ -87,12 +88,12 @@ def time_config(blocks, dx: float, precision: int, cfg: int, steps: int = 3, war
 
 def tune(classes=None, configs=None, precisions=("fp64", "mixed"), steps: int = 3, fp64_chi: float = 0.5,
          device: int = 0, target_points: int = 1 << 21, margin: float = 0.01, log=None) -> dict:
-    """Time every configuration for every class and precision; returns the
+    """Time a configuration of each tile set for every class and precision; returns the
     table (per class the fastest configuration, or configuration 0 unless the
     fastest beats it by more than `margin`; classes not tuned keep None) and
     the timings in ns per point-stage."""
     classes = list(STAGE_CLASS_EDGES if classes is None else classes)
-    configs = list(range(STAGE_CONFIGS) if configs is None else configs)
+    configs = list(STAGE_TILE_SET_CONFIGS if configs is None else configs)
     table = {p: [None] * len(STAGE_CLASS_EDGES) for p in precisions}
     timings = {p: {} for p in precisions}
     for edge in classes:
@@ -136,7 +137,7 @@ def main(argv=None) -> int:
     ap = argparse.ArgumentParser(description=__doc__, formatter_class=argparse.RawDescriptionHelpFormatter)
     ap.add_argument("--out", default=None, help="write the result (JSON) here")
     ap.add_argument("--classes", default=None, help="comma-separated class edges (default: all)")
-    ap.add_argument("--configs", default=None, help="comma-separated configurations (default: all)")
+    ap.add_argument("--configs", default=None, help="comma-separated configurations (default: one per tile set)")
     ap.add_argument("--precisions", default="fp64,mixed", help="comma-separated: fp64, mixed")
     ap.add_argument("--steps", type=int, default=3)
     ap.add_argument("--fp64-chi", type=float, default=0.5)

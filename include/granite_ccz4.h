@@ -400,12 +400,10 @@ GRANITE_API int granite_ccz4_get_kernel_variant(const void* ctx, int* variant);
 
 /* Per-class configurations of GRANITE_VARIANT_TMA (no counterpart in the
  * reference, whose computeRHS runs one OpenMP loop per block, ccz4.cpp:267-270).
- * GRANITE_STAGE_CONFIGS configuration ids exist (granite_ccz4_stage_config_info:
- * the tile depth, ring slots and shared-memory options of the stage kernel each
- * was a candidate of). The present kernel, whose loads are issued by warps of
- * their own, is faster than every one of them on every block size and runs for
- * all ids; an id chooses its tiles: with x-remainder tiles
- * (granite_ccz4_stage_config_schedule) or without. Every block belongs to the
+ * One kernel runs on one of two tile sets, and a configuration id stands for a
+ * set: ids 0 to 10 for 16 x 4 x 2 tiles throughout, ids 11 to
+ * GRANITE_STAGE_CONFIGS - 1 for the set with x-remainder tiles
+ * (granite_ccz4_stage_config_schedule). Every block belongs to the
  * block-size class whose edge (GRANITE_STAGE_CLASS_EDGES) is nearest on a log
  * scale to the cube root of its interior volume; each (precision, class) may be
  * given a configuration; classes without one take the tiles that suit their
@@ -415,15 +413,22 @@ GRANITE_API int granite_ccz4_get_kernel_variant(const void* ctx, int* variant);
 #define GRANITE_STAGE_CLASSES 6
 #define GRANITE_STAGE_CLASS_EDGES 16, 24, 32, 48, 64, 96
 /* cls: class index (0 .. GRANITE_STAGE_CLASSES - 1) or -1 for every class;
- * cfg: configuration or -1 for the built-in default. */
+ * cfg: configuration or -1 to leave the choice to the library. get: the id set for
+ * the class, or, where the choice is the library's, an id of the tile set that
+ * most committed blocks of the class run in that precision (0 or 12); before there
+ * are any, 0 in FP64 and 12 in mixed precision. */
 GRANITE_API int granite_ccz4_set_stage_config(void* ctx, int precision, int cls, int cfg);
 GRANITE_API int granite_ccz4_get_stage_config(const void* ctx, int precision, int cls, int* cfg);
 /* One configuration for every block and precision (-1: back to the per-class table). */
 GRANITE_API int granite_ccz4_force_stage_config(void* ctx, int cfg);
+/* The kernel an id runs: tiles of 16 x 4 x tile_z points, ring_slots field boxes in
+ * flight per compute warpgroup of the mixed kernels (the FP64 kernels have one
+ * more), the stage input's or the Hessian loop's values in shared memory
+ * (shared_input, shared_hessian: 0). */
 GRANITE_API int granite_ccz4_stage_config_info(int cfg, int* tile_z, int* ring_slots, int* shared_input,
                                                int* shared_hessian);
-/* The rest of a configuration's description: warp_specialized, ctas_per_sm and
- * items_per_barrier, of the kernel it was a candidate of (as above);
+/* The rest: load warps of their own (warp_specialized: 1), ctas_per_sm, field boxes
+ * per wait of a warp (items_per_barrier);
  * x_remainder_tiles = 1 when a block whose x extent is 8 more than a multiple
  * of 16 covers its last 8 columns with 8 x 4 x 4 tiles instead of 16-wide tiles
  * half outside the block. Null outputs are skipped. */

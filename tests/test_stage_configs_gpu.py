@@ -1,19 +1,12 @@
-"""Every configuration of the TMA stage kernel (the autotuner's candidates) and
+"""The tile sets of the TMA stage kernel, what the configuration ids stand for, and
 the per-class configuration table.
 
-Configuration 5 runs the mixed form warp-specialized (stencil warps feed
-algebra warps through shared memory): its derivatives are the same FP32
-values, its algebra the same code, so it is held to the same bounds.
-
-The configurations differ in tile depth, ring depth, resident CTAs per SM and
-where intermediate values live (shared memory or registers / local memory),
-never in arithmetic: in FP64 every configuration must give the results of
-configuration 0 bit for bit, and those equal the oracle (the restatement of
+The sets differ in their tiles alone, never in arithmetic: in FP64 both must give
+the same results bit for bit, and those equal the oracle (the restatement of
 ccz4.cpp:251-935 and main.cpp:306-689, pinned to the compiled reference) with
 the multi-step parity bound. Mixed precision is compared with FP64 at the mixed
-tolerance. A hierarchy whose block-size classes use different configurations
-(several launches per level and stage) must equal the single-configuration run
-bit for bit.
+tolerance. A hierarchy whose block-size classes use different sets (several
+launches per level and stage) must equal the run of one set bit for bit.
 """
 import numpy as np
 import pytest
@@ -25,7 +18,7 @@ from test_parity_gpu import parity
 
 pytestmark = pytest.mark.gpu
 
-CONFIGS = list(range(18))
+CONFIGS = [0, 12]  # one id per tile set
 
 
 @pytest.fixture(scope="module")
@@ -36,8 +29,8 @@ def gb():
 
 @pytest.fixture(scope="module")
 def case(oracle_lib):
-    # partial tiles in x (40 = 16 + 16 + 8: configuration 11 covers the last 8 columns with 8 x 4 x 4
-    # remainder tiles), y (22) and z (18 = 4 x 4 + 2 / 9 x 2)
+    # partial tiles in x (40 = 16 + 16 + 8: 8 x 4 x 4 remainder tiles for the last 8 columns, or
+    # 16-wide tiles half outside), y (22) and, of the remainder tiles, z (18 = 4 x 4 + 2)
     g = Geom((40, 22, 18), (-5.0, -2.75, -2.25), (5.0, 2.75, 2.25))
     u = oracle_lib.init_brill_lindquist(g, [1.0], [[0.12, -0.1, 0.05]], r_floor=0.5 * g.dx[0])
     u = oracle.add_noise(u, 1e-10, 99)
@@ -78,7 +71,7 @@ def test_config_fp64_matches_oracle_and_config0(gb, case, cfg):
 @pytest.mark.parametrize("cfg", CONFIGS)
 def test_config_mixed_close_to_fp64(gb, case, cfg, fp64_chi):
     # FP32 algebra everywhere, or per-tile FP64 where chi < 0.5 (both passes of
-    # the per-tile precision run in this configuration)
+    # the per-tile precision run on this tile set)
     g, u, dt, ref = case
     out = _steps(gb, g, u, dt, 4, gb.PRECISION_MIXED, cfg, fp64_chi)
     parity(out, ref, rtol=2e-5, what=f"config {cfg}, 4 mixed steps, fp64_chi {fp64_chi}")
@@ -87,8 +80,8 @@ def test_config_mixed_close_to_fp64(gb, case, cfg, fp64_chi):
 
 
 def test_per_class_table_on_a_hierarchy(gb, oracle_lib):
-    # blocks of three size classes on two levels; each class gets another
-    # configuration, so a level stage runs as several launches
+    # blocks of three size classes on two levels, one class with x-remainder tiles,
+    # so a level stage runs as several launches
     geoms = [Geom((16, 16, 16), (-4.0, -4.0, -4.0), (0.0, 0.0, 0.0)),
              Geom((40, 32, 16), (0.0, -4.0, -4.0), (10.0, 4.0, 0.0)),
              Geom((16, 16, 16), (-4.0, 0.0, -4.0), (0.0, 4.0, 0.0)),
@@ -133,3 +126,21 @@ def test_per_class_table_on_a_hierarchy(gb, oracle_lib):
     for i in range(len(geoms)):
         parity(bm[i], am[i], rtol=1e-6, what=f"mixed block {i}")
 
+
+
+def test_reported_configuration_is_the_one_that_runs(gb):
+    # the library's choice: remainder tiles where they save enough tiles of the level
+    cls24, cls32 = gb.block_stage_class((24, 24, 24)), gb.block_stage_class((32, 32, 32))
+    for precision, before in ((gb.PRECISION_FP64, 0), (gb.PRECISION_MIXED, 12)):
+        ev = gb.Evolver(gb.CCZ4Params(device=0), gb.VARIANT_TMA)
+        assert [ev.stage_config(precision, k) for k in (cls24, cls32)] == [before, before]
+        ev.set_stage_config(precision, cls32, 3)
+        assert ev.stage_config(precision, cls32) == 3
+        ev.set_stage_config(precision, cls32, -1)
+        assert ev.stage_config(precision, cls32) == before
+        for i, (n, level) in enumerate([(24, 0), (32, 1)]):
+            ev.add_block(gb.GridBlock(i, level, (n, n, n), (-1.0,) * 3, (1.0,) * 3))
+        ev.commit()
+        assert ev.stage_config(precision, cls24) == 12
+        assert ev.stage_config(precision, cls32) == 0
+        ev.close()
