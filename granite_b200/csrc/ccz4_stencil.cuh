@@ -43,7 +43,7 @@ struct StridedAxis {
 // axis<D>(beta) the neighbours along axis D.
 // Offsets in int where every stencil is FP64 (EXACT): one wide multiply-add per
 // neighbour instead of a 64-bit addition chain, 4 % of the FP64 global-load RHS
-// (89x70x61: 335 -> 322 us); the mixed build's pair stencils are 8 % slower so
+// (89x70x61: 331 -> 318 us); the mixed build's pair stencils are 8 % slower so
 // (234 -> 253 us) and keep 64-bit offsets. Four planes of cells always fit an
 // int: 2^29 cells in one plane are 850 GB for a block's nine planes or more.
 template <typename O>

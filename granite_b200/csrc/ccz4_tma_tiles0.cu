@@ -2,7 +2,7 @@
 // (ccz4_kernels.h): 16-wide tiles; also the store epilogue.
 // Three ring slots per mixed warpgroup leave the per-point body's local memory
 // an L1 of over 70 KB; the FP64 kernels have two warpgroups and take four
-// (456 us with three, 448 with four on 128 x 128 x 64 points).
+// (478 us with three, 470 with four on 128 x 128 x 64 points).
 #include "ccz4_stage_tma.cuh"
 
 namespace granite_b200 {

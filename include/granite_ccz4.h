@@ -379,8 +379,9 @@ GRANITE_API int granite_ccz4_profile_get(void* ctx, int kernel_class, double* to
  * and its halo through shared memory with cp.async. In a committed hierarchy the
  * GLOBAL tiles are w x 128/w points with w in {32, 16, 8} chosen per block to
  * leave the fewest idle threads. GRANITE_VARIANT_TMA (the default) runs one
- * persistent CTA per SM that streams every field of a 16x4x4 tile and its
- * 4-cell halo into a ring of shared-memory slots with tensor-map (TMA) loads;
+ * persistent CTA per SM whose load warps stream every field of a 16x4x2 tile (8x4x4
+ * for an x-remainder) and its halo into rings of shared-memory slots with
+ * tensor-map (TMA) loads;
  * blocks it cannot map (odd x extent, fewer than 16 x or 4 y/z interior cells)
  * send their level to GRANITE_VARIANT_GLOBAL. A TMA load that does not complete
  * within its wait limit makes the next granite_ccz4_sync, block download
@@ -461,8 +462,8 @@ GRANITE_API int granite_ccz4_test_withhold_tile_load(void* ctx, int item);
 GRANITE_API int granite_ccz4_set_fp64_chi_threshold(void* ctx, double chi_fp64);
 /* 1: the FP64 pass of the per-tile precision runs on a second stream of the
  * context beside the FP32 pass (they write disjoint tiles); 0 (default): after
- * it. Measured on the binary hierarchy: 67.9 vs 67.2 ms per coarse step, the
- * concurrent FP64 CTAs take SM slots the persistent FP32 pass needs. */
+ * it. Measured on the binary hierarchy: 44.0 vs 43.0 ms per coarse step, the
+ * concurrent FP64 CTAs take SMs the persistent FP32 pass needs. */
 GRANITE_API int granite_ccz4_set_pass_overlap(void* ctx, int on);
 GRANITE_API int granite_ccz4_get_fp64_chi_threshold(const void* ctx, double* chi_fp64);
 
@@ -472,7 +473,7 @@ GRANITE_API int granite_ccz4_get_fp64_chi_threshold(const void* ctx, double* chi
  * the fills after the stages only prolongate and apply the block-local fills;
  * 0 (the default) = the fills copy them (the same values: results are
  * identical). Levels whose interiors overlap (after a regrid) always copy.
- * Measured on the binary hierarchy: 73.4 ms per coarse step with pushes, 66.8
+ * Measured on the binary hierarchy: 45.5 ms per coarse step with pushes, 43.0
  * without; a 16^3 block pushes 87 % of its cells, and the stage kernel's
  * scattered ghost stores cost more than the fill kernel's copies. */
 GRANITE_API int granite_ccz4_set_ghost_push(void* ctx, int on);
