@@ -90,10 +90,15 @@ class PinnedLease {
             c.slots = c.own;
         }
     }
-    // (every copy through the slots has been waited for, also after an error)
+    // Every copy through the slots has been waited for, also after an error: a wait is
+    // refused while another thread captures a stream in the global mode, unless
+    // this thread is in the relaxed one.
     ~PinnedLease() {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
         for (auto e : c_.ev)
             if (e) cudaEventSynchronize(e);
+        cudaThreadExchangeStreamCaptureMode(&mode);
         c_.slots = nullptr;
     }
 

@@ -23,6 +23,7 @@ inline double __dmul_rn(double a, double b) { return a * b; }
 
 enum cudaError_t { cudaSuccess = 0, cudaErrorInvalidValue = 1, cudaErrorMemoryAllocation = 2 };
 enum cudaMemcpyKind { cudaMemcpyHostToDevice = 1, cudaMemcpyDeviceToHost = 2 };
+enum cudaStreamCaptureMode { cudaStreamCaptureModeGlobal = 0, cudaStreamCaptureModeThreadLocal = 1, cudaStreamCaptureModeRelaxed = 2 };
 enum { cudaHostAllocPortable = 1, cudaEventDisableTiming = 2 };
 using cudaStream_t = struct FakeStream*;
 using cudaEvent_t = struct FakeEvent*;
@@ -37,3 +38,4 @@ cudaError_t cudaEventSynchronize(cudaEvent_t);
 cudaError_t cudaMemcpyAsync(void*, const void*, size_t, cudaMemcpyKind, cudaStream_t);
 cudaError_t cudaMemcpy2DAsync(void*, size_t, const void*, size_t, size_t, size_t, cudaMemcpyKind, cudaStream_t);
 cudaError_t cudaStreamSynchronize(cudaStream_t);
+cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode*);

@@ -6,17 +6,21 @@
 #include <dlfcn.h>
 #include <pthread.h>
 
+#include <atomic>
 #include <cerrno>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <new>
+#include <set>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "ccz4_host_copy.h"
 
-static bool copying = false;                            // within a copy:
+static std::atomic<bool> copying{false};                            // within a copy:
 static bool no_threads = false, no_thread_state = false;  // what fails there
 
 extern "C" int pthread_create(pthread_t* t, const pthread_attr_t* a, void* (*f)(void*), void* x) noexcept {
@@ -31,7 +35,11 @@ void operator delete(void* p) noexcept { std::free(p); }
 void operator delete(void* p, size_t) noexcept { std::free(p); }
 
 static bool no_pinned = false, no_events = false, no_copies = false;
+static bool capturing = false;  // another thread captures a stream in the global mode
+static thread_local cudaStreamCaptureMode mode = cudaStreamCaptureModeGlobal;
 static int pinned = 0, events = 0;
+static std::mutex in_flight_m;
+static std::set<cudaEvent_t> in_flight;  // recorded and not waited for
 
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
     if (no_pinned) return cudaErrorMemoryAllocation;
@@ -57,8 +65,24 @@ cudaError_t cudaEventDestroy(cudaEvent_t e) {
     std::free(e);
     return cudaSuccess;
 }
-cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t) {
+    std::lock_guard<std::mutex> l(in_flight_m);
+    const bool was = copying;
+    copying = false;  // (the set's own memory)
+    in_flight.insert(e);
+    copying = was;
+    return cudaSuccess;
+}
+cudaError_t cudaEventSynchronize(cudaEvent_t e) {
+    if (capturing && mode != cudaStreamCaptureModeRelaxed) return cudaErrorInvalidValue;
+    std::lock_guard<std::mutex> l(in_flight_m);
+    in_flight.erase(e);
+    return cudaSuccess;
+}
+cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode* m) {
+    std::swap(*m, mode);
+    return cudaSuccess;
+}
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
     if (no_copies) return cudaErrorInvalidValue;
     std::memcpy(d, s, n);
@@ -116,6 +140,19 @@ int main(int argc, char** argv) {
             bad += copy_in(c, b.data(), a.data(), a.size() * sizeof(double), nullptr) == cudaSuccess;
             bad += copy_out_interior(c, b.data(), a.data(), small, 22, nullptr) == cudaSuccess;
         }
+        c.destroy();
+    }
+    if (what == "capture_elsewhere") {  // the call fails, but hands the slots on with no copy in flight
+        capturing = true;
+        std::vector<double> a(1 << 20), b(1 << 20);
+        HostCopy c;
+        c.create(0);
+        {
+            PinnedLease lease(c);
+            bad += copy_in(c, b.data(), a.data(), a.size() * sizeof(double), nullptr) == cudaSuccess;
+            bad += in_flight.empty();
+        }
+        bad += !in_flight.empty() || mode != cudaStreamCaptureModeGlobal;
         c.destroy();
     }
     std::printf(bad ? "%d wrong\n" : "OK\n", bad);

@@ -39,7 +39,8 @@ def test_every_kernel_answers_for_its_registers(tmp_path):
     assert r.returncode == 0, r.stdout + r.stderr
 
 
-@pytest.mark.parametrize("what", ["staged", "no_pinned", "no_events", "no_threads", "no_thread_state", "copy_error"])
+@pytest.mark.parametrize("what", ["staged", "no_pinned", "no_events", "no_threads", "no_thread_state", "copy_error",
+                                  "capture_elsewhere"])
 def test_host_copies(tmp_path, what):
     r = subprocess.run([build(tmp_path, "test_host_copy"), what], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout + r.stderr
